@@ -199,7 +199,7 @@ int fixed_point_shift(double bound)
 }
 
 // form: two-word exact words (FP64 form) or one signed word (FP32 form,
-// flush.cuh:warp_drain_nodes); both keep every bin total inside the word's range
+// flush.cuh:warp_drain32); both keep every bin total inside the word's range
 void set_shifts(galic_ctx *ctx, int *shift, int form)
 {
   const galic_params_t &p = ctx->prm;
@@ -826,9 +826,9 @@ int enqueue_orbits(galic_ctx *ctx, int form, int first, int stride, int *launche
 }
 
 // fixed point -> committed grids, then calc_global_fit (main.c:251-362)
-int enqueue_finish(galic_ctx *ctx, int *launches)
+int enqueue_finish(galic_ctx *ctx, int form, int *launches)
 {
-  launch_fx_finalize(ctx->d_fx, ctx->d_shift, ctx->d_committed, 4 * NG_COMMITTED, ctx->G, ctx->stream);
+  launch_fx_finalize(ctx->d_fx, ctx->d_shift, ctx->d_committed, 4 * NG_COMMITTED, ctx->G, form, ctx->stream);
   *launches += 1;
   *launches += launch_global_fit(make_fit_args(ctx), ctx->stream);
   CK(cudaGetLastError());
@@ -878,7 +878,7 @@ extern "C" int galic_calc_all_response_fields(galic_ctx *ctx, int form)
   if(st) return st;
   int launches = 0;
   if((st = enqueue_orbits(ctx, form, 0, 1, &launches))) return st;
-  if((st = enqueue_finish(ctx, &launches))) return st;
+  if((st = enqueue_finish(ctx, form, &launches))) return st;
   if((st = collect(ctx, launches, true))) return st;
   ctx->have_response = true;
   return fail(ctx, GALIC_OK);
@@ -910,7 +910,7 @@ extern "C" int galic_calc_all_finish(galic_ctx *ctx)
   if(!ctx) return GALIC_ERR_INVALID_ARGUMENT;
   if(ctx->shard_form < 0) return fail(ctx, GALIC_ERR_STATE);
   int launches = 0;
-  int st = enqueue_finish(ctx, &launches);
+  int st = enqueue_finish(ctx, ctx->shard_form, &launches);
   if(st) return st;
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->last_launches = launches;

@@ -127,7 +127,7 @@ int enqueue_iteration(galic_ensemble *e, int variant, int grid)
     FxWord *fx = e->d_fx + (size_t) m * 4 * NG_COMMITTED * e->G;
     const int *shift = e->d_shift + m * 4 * NG_COMMITTED;
     launch_instantaneous(c->dm, c->n, c->d_pos, c->d_vel, c->d_mass, c->d_type, c->d_vdisp, fx, shift, e->G, s);
-    launch_fx_finalize(fx, shift, c->d_committed, 4 * NG_COMMITTED, e->G, s);
+    launch_fx_finalize(fx, shift, c->d_committed, 4 * NG_COMMITTED, e->G, GALIC_FORM_FP32, s);
     launch_global_fit(make_fit_args(c), s);
   }
   ECK(cudaGetLastError());

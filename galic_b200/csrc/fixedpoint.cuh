@@ -22,6 +22,13 @@ struct FxWord {
   unsigned long long lo;  // sum of L
 };
 
+// The FP32 form's time-averaged accumulators of one grid node: one signed
+// word per field (of scale 2^(S-24)), the other five unused, so that a set's
+// nodes fill the space of its five grids of word pairs.
+struct FxNode32 {
+  unsigned long long w[5], unused[5];
+};
+
 __device__ __forceinline__ void fx_split(double v, int S, long long *H, unsigned long long *L)
 {
   double t = ldexp(v, S - 24);  // exact power-of-two scaling

@@ -52,7 +52,7 @@ struct CalcAllArgs {
   const int *type;
   const int *order;           // processing order (longest first)
   int *next;                  // work counter, zeroed by the caller
-  FxWord *fx;                 // [4][NG_COMMITTED][Ngrid]
+  FxWord *fx;                 // [4][NG_COMMITTED][Ngrid] (FP32: time-averaged half as FxNode32 [4][2][Ngrid])
   const int *shift;           // [4][NG_COMMITTED]
   int *orbits;                // per particle
   unsigned long long *steps_total;
@@ -84,7 +84,8 @@ int launch_calc_all_fp64(const DevModel &M, const CalcAllArgs &a, int grid, int 
 void launch_instantaneous(const DevModel &M, int n, const double *pos, const double *vel, const double *mass,
                           const int *type, double *vdisp, FxWord *fx, const int *shift, int Ngrid, cudaStream_t s,
                           int first = 0, int stride = 1);
-void launch_fx_finalize(const FxWord *fx, const int *shift, double *committed, int count, int Ngrid, cudaStream_t s);
+void launch_fx_finalize(const FxWord *fx, const int *shift, double *committed, int count, int Ngrid, int form,
+                        cudaStream_t s);
 int launch_global_fit(const FitArgs &f, cudaStream_t s);
 cudaError_t prepare_fit_kernels();
 int calc_all_occupancy(int block);

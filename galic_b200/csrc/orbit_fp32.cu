@@ -253,7 +253,7 @@ struct Sink32 : NodeAcc {
 #pragma unroll
     for(int s = 0; s < 4; s++) {
       if(rec[s]) {
-        q->base[at[s]][lane] = (cur_iz + node_dz(s, cur_iz)) * Nb + cur_iR + node_dr(s, cur_iR);
+        q->base[at[s]][lane] = (unsigned short) ((cur_iz + node_dz(s, cur_iz)) * Nb + cur_iR + node_dr(s, cur_iR));
 #pragma unroll
         for(int f = 0; f < 5; f++) q->val[at[s]][f][lane] = a[s][f];
       }
@@ -577,7 +577,7 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
     {
       const int gs = S.gridset(mi, type);
       const double fac = P.mass[p] / P.tint[p];
-      sink.set_orbit(gs * NG_COMMITTED * G, (float) ldexp(fac, S.shift[gs * NG_COMMITTED + GALIC_GRID_MASS_S] - 24),
+      sink.set_orbit(2 * gs * G, (float) ldexp(fac, S.shift[gs * NG_COMMITTED + GALIC_GRID_MASS_S] - 24),
                      (float) ldexp(fac, S.shift[gs * NG_COMMITTED + GALIC_GRID_R_S] - 24));
     }
     sink.cur = -1;
@@ -598,7 +598,7 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
     // records carry the orbit's grid set and scale only through the lane's
     // queue header, so a lane drains them before it starts the next orbit
     if(queue32_due<PER>(sink.cnt) || __any_sync(0xffffffffu, (all_done || state == LANE_START) && sink.cnt > 0))
-      warp_drain32(*sink.q, S.fx, G, sink.cnt);
+      warp_drain32(*sink.q, (FxNode32 *) S.fx, sink.cnt);
     if(all_done) break;
     if(state == LANE_ACTIVE) {
       if(!orbit32_step<Sink32<PER>, true>(S.model(mi), s, sink)) state = s.status == ORBIT_OK ? LANE_LAST : LANE_FINISH;

@@ -130,12 +130,12 @@ __global__ void k_scale_dense(OrbitBatch b, int G)
 // parities, and when the orbit moves to a neighbouring cell the nodes the two
 // cells share stay in place.  Only the slots whose node leaves are parked, as
 // records {node index, 5 sums}, in the lane's column of the warp's queue; the
-// warp drains all lanes' records together (flush.cuh:warp_drain_nodes_exact),
+// warp drains all lanes' records together (flush.cuh:warp_drain64),
 // each value scaled by mass/Tint and added as an exact two-word fixed-point
 // pair (order independent).
 template <int PER>
 struct NodeSink64 {
-  WarpQueueT<PER, double> *q;
+  WarpQueue64<PER> *q;
   int lane, Nb;
   int cnt;  // records parked in this lane's column since the last drain
   int cur_iR, cur_iz;  // the current cell; cur_iz < 0: none
@@ -241,7 +241,7 @@ constexpr int kPer64 = 8;
 template <int MINB>
 __global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(DevModel M, CalcAllArgs A)
 {
-  __shared__ WarpQueueT<kPer64, double> queues[CALC_ALL_BLOCK_FP64 / 32];
+  __shared__ WarpQueue64<kPer64> queues[CALC_ALL_BLOCK_FP64 / 32];
   // the CTA's step count, largest energy error (as bits: non-negative
   // doubles order like them) and worst status, added to at each orbit's end
   // instead of being held in every thread's registers
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(Dev
     // header: a lane's records are drained before it starts the next orbit
     if(queue32_due<kPer64>(sink.cnt) ||
        __any_sync(0xffffffffu, (all_done || state == LANE_START) && sink.cnt > 0))
-      warp_drain_nodes_exact(*sink.q, A.fx, G, sink.cnt);
+      warp_drain64(*sink.q, A.fx, G, sink.cnt);
     if(all_done) break;
     if(state == LANE_ACTIVE) {
       if(!orbit_step(M, L, s, true, sink)) state = LANE_FINISH;
@@ -346,12 +346,20 @@ __global__ void k_instantaneous(DevModel M, int n, int first, int stride, const 
   }
 }
 
-__global__ void k_fx_finalize(const FxWord *fx, const int *shift, double *out, int count, int Ngrid)
+// fp32: the time-averaged grids of every set hold its FxNode32 words
+__global__ void k_fx_finalize(const FxWord *fx, const int *shift, double *out, int count, int Ngrid, bool fp32)
 {
   size_t total = (size_t) count * Ngrid;
   for(size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < total; i += (size_t) gridDim.x * blockDim.x) {
     int g = (int) (i / Ngrid);
-    out[i] = fx_value(fx[i], shift[g]);
+    FxWord w = fx[i];
+    if(fp32 && g % NG_COMMITTED < NF_ORBIT) {
+      // the first five grids of a set are half of its NG_COMMITTED
+      const FxNode32 *nodes = (const FxNode32 *) fx + (size_t) (g / NG_COMMITTED) * 2 * Ngrid;
+      w.hi = nodes[i % Ngrid].w[g % NG_COMMITTED];
+      w.lo = 0;
+    }
+    out[i] = fx_value(w, shift[g]);
   }
 }
 
@@ -395,10 +403,11 @@ void launch_instantaneous(const DevModel &M, int n, const double *pos, const dou
                                                       Ngrid);
 }
 
-void launch_fx_finalize(const FxWord *fx, const int *shift, double *committed, int count, int Ngrid, cudaStream_t s)
+void launch_fx_finalize(const FxWord *fx, const int *shift, double *committed, int count, int Ngrid, int form,
+                        cudaStream_t s)
 {
   size_t total = (size_t) count * Ngrid;
   int grid = (int) ((total + 255) / 256);
   if(grid > 148 * 8) grid = 148 * 8;
-  k_fx_finalize<<<grid, 256, 0, s>>>(fx, shift, committed, count, Ngrid);
+  k_fx_finalize<<<grid, 256, 0, s>>>(fx, shift, committed, count, Ngrid, form == GALIC_FORM_FP32);
 }
