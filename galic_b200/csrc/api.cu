@@ -199,7 +199,7 @@ int fixed_point_shift(double bound)
 }
 
 // form: two-word exact words (FP64 form) or one signed word (FP32 form,
-// flush.cuh:warp_drain32); both keep every bin total inside the word's range
+// flush.cuh:add_field); both keep every bin total inside the word's range
 void set_shifts(galic_ctx *ctx, int *shift, int form)
 {
   const galic_params_t &p = ctx->prm;

@@ -22,11 +22,11 @@ struct FxWord {
   unsigned long long lo;  // sum of L
 };
 
-// The FP32 form's time-averaged accumulators of one grid node: one signed
-// word per field (of scale 2^(S-24)), the other five unused, so that a set's
-// nodes fill the space of its five grids of word pairs.
-struct FxNode32 {
-  unsigned long long w[5], unused[5];
+// The time-averaged accumulators of one grid node: the five fields' H words,
+// then their L words; the FP32 form uses the first five words only, one
+// signed word per field.  A set's nodes fill the space of its five grids.
+struct FxNode {
+  unsigned long long hi[5], lo[5];
 };
 
 __device__ __forceinline__ void fx_split(double v, int S, long long *H, unsigned long long *L)
@@ -49,26 +49,12 @@ __device__ __forceinline__ void fx_split(double v, int S, long long *H, unsigned
 // power-of-two factor is exact, so the pair equals fx_split's)
 __device__ __forceinline__ void fx_split_scaled(double t, long long *H, unsigned long long *L)
 {
-  double fh = floor(t);
-  double fr = t - fh;
-  long long h = (long long) fh;
-  unsigned long long l = (unsigned long long) rint(fr * 16777216.0);
-  if(l == 16777216ULL) {
-    l = 0;
-    h += 1;
-  }
-  *H = h;
-  *L = l;
-}
-
-__device__ __forceinline__ void fx_add_scaled(FxWord *w, double t)
-{
-  if(t == 0.0) return;
-  long long H;
-  unsigned long long L;
-  fx_split_scaled(t, &H, &L);
-  if(H) atomicAdd(&w->hi, (unsigned long long) H);
-  if(L) atomicAdd(&w->lo, L);
+  const double fh = floor(t);
+  const double fr = t - fh;
+  // rint(fr 2^24), 0 .. 2^24: the low word of its sum with 2^52
+  const unsigned l = (unsigned) __double2loint(fr * 16777216.0 + 4503599627370496.0);
+  *H = (long long) fh + (l >> 24);
+  *L = l & 0xffffffu;
 }
 
 // adds v to the word pair w (no return value needed: red.global.add.u64)

@@ -8,11 +8,45 @@
 // could pass PER; the drain takes all lanes' records together, so that the
 // global atomics run on full warps.  PER is chosen per block size so that the
 // queues fit the static shared memory.
+//
+// A drain hands each record to five neighbouring lanes, one field each (six
+// records a round, lanes 30 and 31 idle).  A node's words are contiguous
+// (fixedpoint.cuh:FxNode), so one atomic instruction covers runs of five words,
+// two sectors a record: L2 executes atomics by sector (a B200 does 1.85e11 /s
+// of random isolated words, 4 to 5e11 words/s in runs of five), and the L1
+// passes them on by sector too.  Measured on the halo + disk pass (1.2e6
+// orbits, 4.8e9 orbit-steps, 1.3 records each), orbit kernel: FP32 156 ms with
+// a record per lane and a grid per field, 141 ms so (126 ms without the
+// atomics, 95 ms without the drain); FP64 324 and 300 ms (its L1 data stage
+// 69 % and 58 % busy).  Other forms, FP64: ten lanes a record, one word each,
+// 391 ms (half the conversions are redundant); two or four rounds unrolled 385
+// and 323 ms; a record per lane, staged in shared memory and added by the copy
+// engine's bulk reductions, 344 ms (the engine adds 6.2e10 records/s, but each
+// lane's command and its proxy fence hold up the warp).
 #ifndef GALIC_FLUSH_CUH
 #define GALIC_FLUSH_CUH
 
 #include "fixedpoint.cuh"
 #include "kernels.cuh"
+
+// T: the type of the sums (float, double)
+template <int PER_, class T>
+struct WarpQueueT {
+  static constexpr int PER = PER_;
+  static_assert(PER_ * 32 <= 256, "list entries are bytes");
+  T val[PER][5][33];             // the node's five sums (33: the five lanes of a record read distinct banks)
+  T scale[2][32];                // per lane: {mass field, energy fields} fixed-point factors
+  int gbase[32];                 // per lane: first node of its orbit's grid set
+  unsigned short base[PER][32];  // the node's index in its grid
+  unsigned char list[PER * 32];  // drain: the parked records, slot * 32 + lane
+};
+template <int PER>
+using WarpQueue32 = WarpQueueT<PER, float>;
+template <int PER>
+using WarpQueue64 = WarpQueueT<PER, double>;
+
+// records per lane of a block of BLOCK threads (FP32 sums)
+__host__ __device__ constexpr int queue32_per(int block) { return block <= 128 ? 8 : (block <= 192 ? 7 : 5); }
 
 // true when some lane could not park another cell's nodes
 template <int PER>
@@ -21,41 +55,33 @@ __device__ __forceinline__ bool queue32_due(int cnt)
   return __any_sync(0xffffffffu, cnt > PER - 4);
 }
 
-// ---------------------------------------------------------------- FP32 sums
+// FP32 sums: value x 2^(shift-24) (the orbit's mass/Tint and the field's
+// fixed-point scale folded into one FP32 factor per field class when the
+// orbit starts) rounded to one signed 64-bit word.  shift - 24 is chosen so
+// that no bin can overflow 2^62; the FP32 rounding of the scaled value (2^-24
+// relative) is far inside the FP32 form's tolerance.
+__device__ __forceinline__ void add_field(FxNode *n, int f, float t)
+{
+  const long long X = __float2ll_rn(t);
+  if(X) atomicAdd(&n->hi[f], (unsigned long long) X);
+}
+// FP64 sums: the two-word pair of v = sum x mass/Tint (resolution 2^-S), so
+// that the bins carry the full FP64 resolution whatever the headroom of the
+// field's range.  The factor is mass/Tint x 2^(S-24), whose power of two is
+// exact, so the pair is fx_split(v, S)'s bit for bit.
+__device__ __forceinline__ void add_field(FxNode *n, int f, double t)
+{
+  long long H;
+  unsigned long long L;
+  fx_split_scaled(t, &H, &L);
+  atomicAdd(&n->hi[f], (unsigned long long) H);
+  atomicAdd(&n->lo[f], L);
+}
 
-template <int PER_>
-struct WarpQueue32 {
-  static constexpr int PER = PER_;
-  static_assert(PER_ * 32 <= 256, "list entries are bytes");
-  float val[PER][5][33];         // the node's five sums (33: the five lanes of a record read distinct banks)
-  float scale[2][32];            // per lane: {mass field, energy fields} fixed-point factors
-  int gbase[32];                 // per lane: first node of its orbit's grid set
-  unsigned short base[PER][32];  // the node's index in its grid
-  unsigned char list[PER * 32];  // drain: the parked records, slot * 32 + lane
-};
-
-// records per lane of a block of BLOCK threads
-__host__ __device__ constexpr int queue32_per(int block) { return block <= 128 ? 8 : (block <= 192 ? 7 : 5); }
-
-// Every value is scaled by 2^(shift-24) mass/Tint (one FP32 factor per field
-// class, formed when the orbit starts) and rounded to one signed 64-bit word.
-// shift - 24 is chosen so that no bin can overflow 2^62; the FP32 rounding of
-// the scaled value (2^-24 relative) is far inside the FP32 form's tolerance.
-//
-// The words are stored node by node (fixedpoint.cuh:FxNode32), and a record
-// is handed to five neighbouring lanes, one field each (six records at a
-// time, lanes 30 and 31 idle): one atomic instruction then covers runs of
-// five consecutive words, 2-3 sectors a record.  L2 executes atomics by
-// sector (a B200 does 1.85e11 /s of random isolated words, 4 to 5e11 words/s
-// in runs of five).  With a record per lane and field-major grids, five
-// isolated words a record, the halo + disk pass of 1.2e6 orbits (4.8e9
-// orbit-steps, 1.3 records each) ran 156 ms; so it runs 141 ms (126 ms
-// without the atomics, 95 ms without the drain).
-//
-// All 32 lanes call this at the same point of the loop with their record
-// counts; cnt is 0 on return.
-template <int PER>
-__device__ __forceinline__ void warp_drain32(WarpQueue32<PER> &q, FxNode32 *fx, int &cnt)
+// all 32 lanes call this at the same point of the loop with their record
+// counts; cnt is 0 on return
+template <int PER, class T>
+__device__ __forceinline__ void warp_drain_nodes(WarpQueueT<PER, T> &q, FxNode *fx, int &cnt)
 {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -74,60 +100,7 @@ __device__ __forceinline__ void warp_drain32(WarpQueue32<PER> &q, FxNode32 *fx, 
   const int grp = lane / 5, f = lane - 5 * grp;
   for(int r = lane < 30 ? grp : total; r < total; r += 6) {
     const int e = q.list[r], k = e >> 5, l = e & 31;
-    const long long X = __float2ll_rn(q.val[k][f][l] * q.scale[f ? 1 : 0][l]);
-    if(X) atomicAdd(&fx[q.gbase[l] + q.base[k][l]].w[f], (unsigned long long) X);
-  }
-  __syncwarp();
-  cnt = 0;
-}
-
-// ---------------------------------------------------------------- FP64 sums
-
-template <int PER_>
-struct WarpQueue64 {
-  static constexpr int PER = PER_;
-  int base[PER][32];       // the node's index in its grid (field f of the orbit's set: gbase + f * Ngrid + base)
-  double val[PER][5][32];  // the node's five sums
-  int off[32];             // drain: first compacted record of each lane
-  int gbase[32];           // per lane: first word of its orbit's grid set
-  double scale[2][32];     // per lane: {mass field, energy fields} fixed-point factors
-};
-
-// Every value v = sum x mass/Tint is added as the two-word fixed-point pair
-// of fixedpoint.cuh:fx_add (resolution 2^-S, two integer atomics), so the bins
-// carry the full FP64 resolution whatever the headroom of the field's range.
-// The lane header holds mass/Tint x 2^(S-24) per field class (scale), which
-// gives the pair of fx_add(v, S) bit for bit: the power-of-two factor is
-// exact.  A record per lane here: its five conversions overlap.  Five lanes
-// per record with node-major words, as above, ran 584 ms against 378 ms (the
-// conversions become a serial chain per round; 475 ms with four rounds
-// unrolled), a record per lane with node-major pairs 440 ms (the lanes of one
-// atomic instruction then touch 32 lines).
-template <int PER>
-__device__ __forceinline__ void warp_drain64(WarpQueue64<PER> &q, FxWord *fx, int G, int &cnt)
-{
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  int incl = cnt;
-#pragma unroll
-  for(int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(FULL, incl, o);
-    if(lane >= o) incl += y;
-  }
-  const int total = __shfl_sync(FULL, incl, 31);
-  q.off[lane] = incl - cnt;
-  __syncwarp();
-  for(int r = lane; r < total; r += 32) {
-    // the lane L whose records hold r: the last L with off[L] <= r
-    int L = 0;
-#pragma unroll
-    for(int step = 16; step; step >>= 1)
-      if(q.off[L + step] <= r) L += step;
-    const int k = r - q.off[L];
-    const int b = q.gbase[L] + q.base[k][L];
-    const double sm = q.scale[0][L], se = q.scale[1][L];
-#pragma unroll
-    for(int f = 0; f < 5; f++) fx_add_scaled(&fx[b + f * G], q.val[k][f][L] * (f == 0 ? sm : se));
+    add_field(&fx[q.gbase[l] + q.base[k][l]], f, q.val[k][f][l] * q.scale[f ? 1 : 0][l]);
   }
   __syncwarp();
   cnt = 0;

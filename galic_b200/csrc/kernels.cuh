@@ -18,9 +18,11 @@ enum { NG_COMMITTED = 10 };
 #define CALC_ALL_BLOCK_FP64 128
 #define CALC_ALL_BLOCK_FP32 128
 #ifndef GALIC_FP64_MIN_BLOCKS
-// 4 CTAs of 128 threads per SM (128 registers, a few spilled) ran the
-// halo + disk pass 10 % faster than 3 CTAs at 156 registers
-#define GALIC_FP64_MIN_BLOCKS 4
+// 3 CTAs of 128 threads per SM (158 registers, none spilled) run the halo +
+// disk pass in 300 ms; 4 CTAs (128 registers, 110 bytes spilled) take 363 ms and
+// 2 CTAs 302 ms: past 2 warps per scheduler the L1 data stage, the issue slots
+// and the FP64 pipe (72, 66 and 50 % busy) share the limit
+#define GALIC_FP64_MIN_BLOCKS 3
 #endif
 #ifndef GALIC_FP32_MIN_BLOCKS
 // 5 CTAs per SM (96 registers, none spilled; 5 x 31 KiB of queues) ran the
@@ -52,7 +54,7 @@ struct CalcAllArgs {
   const int *type;
   const int *order;           // processing order (longest first)
   int *next;                  // work counter, zeroed by the caller
-  FxWord *fx;                 // [4][NG_COMMITTED][Ngrid] (FP32: time-averaged half as FxNode32 [4][2][Ngrid])
+  FxWord *fx;                 // [4][NG_COMMITTED][Ngrid] (the time-averaged five of a type as FxNode[Ngrid])
   const int *shift;           // [4][NG_COMMITTED]
   int *orbits;                // per particle
   unsigned long long *steps_total;

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "gmath.h"
+#include "stepmath.cuh"
 
 #define GALIC_STEP_CAP 100000000LL  // orbit_response.c:450
 
@@ -36,6 +37,7 @@ struct DevModel {
   // log(FG_Fac), log(DG_Fac) (set_step_constants)
   double lfg, ldg, leg;
   double inv_FG_Rmin, inv_DG_Rmin, inv_lfg, inv_ldg;
+  int step_ok;  // the step's per-model operands are in stepmath.cuh's ranges
   // tables (device pointers, reference layouts)
   const double2 *fg_acc;  // {FG_DPotDR, FG_DPotDz}[iz*FG_Nbin+iR]
   const double *fg_pot;
@@ -56,6 +58,9 @@ inline void set_step_constants(DevModel &M)
   M.inv_DG_Rmin = 1.0 / M.DG_Rmin;
   M.inv_lfg = 1.0 / M.lfg;
   M.inv_ldg = 1.0 / M.ldg;
+  const double lo = 0x1.0p-100, hi = 0x1.0p+100;
+  M.step_ok = M.FG_Rmin >= lo && M.FG_Rmin <= hi && M.DG_Rmin >= lo && M.DG_Rmin <= hi && M.V200 >= lo && M.V200 <= hi &&
+              M.lfg >= 0x1.0p-20 && M.ldg >= 0x1.0p-20;
 }
 
 // a / b for a divisor b fixed per model, given y = 1/b correctly rounded:
@@ -352,41 +357,37 @@ __device__ __forceinline__ double get_timestep(const DevModel &M, const double *
   return t1 < t2 ? t1 : t2;  // dmin, system.c:46
 }
 
-// One deposit of orbit_response.c:277-320: the weights m[a][b] of the four
-// corners of cell k, and the projections.
-struct Deposit {
-  int iR, iz;
-  double m00, m10, m01, m11;
-  Proj p;
-};
-__device__ __forceinline__ Deposit make_deposit(double dt, const Cell &k, const Proj &p)
-{
-  Deposit d;
-  d.iR = k.iR;
-  d.iz = k.iz;
-  d.m00 = 0.5 * dt * (1 - k.fR) * (1 - k.fz);
-  d.m10 = 0.5 * dt * (k.fR) * (1 - k.fz);
-  d.m01 = 0.5 * dt * (1 - k.fR) * (k.fz);
-  d.m11 = 0.5 * dt * (k.fR) * (k.fz);
-  d.p = p;
-  return d;
-}
+// The weights of orbit_response.c:277-320 for the four corners of cell k and
+// the half step hdt = 0.5 dt: corner (dz, dr) gets
+// hdt * (dr ? fR : 1 - fR) * (dz ? fz : 1 - fz).
 
 // Orbit state of produce_orbit_response_field_mod (orbit_response.c:170-209)
+// between two steps: the coming step's dt is set and its first half deposit
+// made.
 struct OrbitState {
   double x[3], v[3], a[3];
-  double tall, timespan, E0;
+  double dt, tall, timespan, E0;
   bool rad_in;  // radsign_previous < 0: all the reference reads of it
-  Cell cell;
-  Proj proj;
   long long steps;
   int norbit, flag, type, tovs, status;
 };
 
+// the time step limited to the time span (orbit_response.c:213-220)
+__device__ __forceinline__ void set_step(OrbitState &s, double dt)
+{
+  if(0 < s.timespan)
+    if(s.timespan < dt + s.tall) {
+      dt = s.timespan - s.tall;
+      s.flag = 1;
+    }
+  s.dt = dt;
+}
+
 // orbit_response.c:181-209: copy the initial state, first acceleration, cell,
-// projections and energy
+// projections and energy; the first step's dt and first half deposit
+template <class Sink>
 __device__ __forceinline__ void orbit_begin(const DevModel &M, const LogConsts &L, OrbitState &s, const double *pos,
-                                            const double *vel, double timespan, int type, bool with_proj)
+                                            const double *vel, double timespan, int type, bool with_proj, Sink &sink)
 {
   for(int i = 0; i < 3; i++) {
     s.x[i] = pos[i];
@@ -403,60 +404,210 @@ __device__ __forceinline__ void orbit_begin(const DevModel &M, const LogConsts &
   s.status = ORBIT_OK;
   FgCoord fc = fg_coord(M, L, s.x);
   forcegrid_acc(M, fc, s.x, s.a);
-  s.cell = density_cell(M, L, s.x);
+  const Cell cell = density_cell(M, L, s.x);
   s.E0 = 0.5 * (s.v[0] * s.v[0] + s.v[1] * s.v[1] + s.v[2] * s.v[2]) + forcegrid_pot(M, L, s.x);
-  if(with_proj) s.proj = project(M, s.tovs, type, fc, s.x, s.v, sqrt(s.x[0] * s.x[0] + s.x[1] * s.x[1]));
+  Proj proj{};
+  if(with_proj) proj = project(M, s.tovs, type, fc, s.x, s.v, sqrt(s.x[0] * s.x[0] + s.x[1] * s.x[1]));
+  set_step(s, get_timestep(M, s.v, s.a, cell.iz * M.DG_Nbin + cell.iR));
+  sink.enter(cell.iR, cell.iz);
+  sink.add(cell, 0.5 * s.dt, 0.0, proj);
+}
+
+// What one position gives: the acceleration, the density-grid cell, the
+// force-grid coordinates and R
+struct Place {
+  double a[3], Rxy;
+  FgCoord fc;
+  Cell cell;
+  double cs;  // place_fast: DG_CellSize of the cell
+};
+struct Vec3 {
+  double c[3];
+};
+// any position (the general functions; arguments and results by value, so
+// that the step's own state keeps to registers)
+__device__ __noinline__ static Place place_general(const DevModel &M, Vec3 xv)
+{
+  const LogConsts L = step_log_consts(M);
+  const double *x = xv.c;
+  Place P;
+  P.Rxy = sqrt(x[0] * x[0] + x[1] * x[1]);
+  const double az = gm_fabs(x[2]);
+  P.fc.jdbl = div_by(gm_log(div_by(P.Rxy, M.FG_Rmin, M.inv_FG_Rmin) + 1.0), L.lfg, M.inv_lfg);
+  P.fc.idbl = div_by(gm_log(div_by(az, M.FG_Rmin, M.inv_FG_Rmin) + 1.0), L.lfg, M.inv_lfg);
+  const double ld0 = gm_log(div_by(P.Rxy, M.DG_Rmin, M.inv_DG_Rmin) + 1.0);
+  const double ld1 = gm_log(div_by(az, M.DG_Rmin, M.inv_DG_Rmin) + 1.0);
+  forcegrid_acc(M, P.fc, x, P.a);
+  P.cell = cell_from_b(div_by(ld0, L.ldg, M.inv_ldg) - 0.5, div_by(ld1, L.ldg, M.inv_ldg) - 0.5, M.DG_Nbin);
+  return P;
+}
+
+// cell_from_b for finite br, bz < 2^31
+__device__ __forceinline__ Cell step_cell(double br, double bz, int nbin)
+{
+  Cell c;
+  br = br < 0 ? 0.0 : br;
+  bz = bz < 0 ? 0.0 : bz;
+  const StepFloor r = step_floor(br), z = step_floor(bz);
+  const bool in_r = r.i < nbin - 1, in_z = z.i < nbin - 1;
+  c.iR = in_r ? r.i : nbin - 2;
+  c.iz = in_z ? z.i : nbin - 2;
+  c.fR = in_r ? br - r.d : 1.0;
+  c.fz = in_z ? bz - z.d : 1.0;
+  return c;
+}
+
+// the same results for a position whose components step_safe accepts (false
+// otherwise: P is not valid)
+__device__ __forceinline__ bool place_fast(const DevModel &M, const LogConsts &L, const double *x, Place &P)
+{
+  if(!M.step_ok || !step_safe(x)) return false;
+  P.Rxy = step_sqrt(x[0] * x[0] + x[1] * x[1]);
+  const double az = gm_fabs(x[2]);
+  // the four log coordinates of the new position (force grid: grid.c:130-136;
+  // density grid: grid.c:494-534)
+  const double lf0 = step_log(div_by(P.Rxy, M.FG_Rmin, M.inv_FG_Rmin) + 1.0);
+  const double lf1 = step_log(div_by(az, M.FG_Rmin, M.inv_FG_Rmin) + 1.0);
+  const double ld0 = step_log(div_by(P.Rxy, M.DG_Rmin, M.inv_DG_Rmin) + 1.0);
+  const double ld1 = step_log(div_by(az, M.DG_Rmin, M.inv_DG_Rmin) + 1.0);
+  P.fc.jdbl = div_by(lf0, L.lfg, M.inv_lfg);
+  P.fc.idbl = div_by(lf1, L.lfg, M.inv_lfg);
+  P.cell = step_cell(div_by(ld0, L.ldg, M.inv_ldg) - 0.5, div_by(ld1, L.ldg, M.inv_ldg) - 0.5, M.DG_Nbin);
+  // the table loads (indices clamped into the table) before the azimuth's
+  // arithmetic, which covers them: the force grid's cells come from L2
+  P.cs = __ldg(&M.cellsize[P.cell.iz * M.DG_Nbin + P.cell.iR]);
+  const int N = M.FG_Nbin;
+  const StepFloor j = step_floor(P.fc.jdbl), i = step_floor(P.fc.idbl);
+  const double2 *T = M.fg_acc + min(i.i, N - 2) * N + min(j.i, N - 2);
+  const double2 t00 = __ldg(&T[0]), t01 = __ldg(&T[1]), t10 = __ldg(&T[N]), t11 = __ldg(&T[N + 1]);
+  double sp, cp;
+  unsigned ones = 0;
+  step_direction(x[1], x[0], &sp, &cp, ones);
+  // forcegrid_get_acceleration (grid.c:122-197)
+  if(M.tabulated) {
+    if(j.i < N - 1 && i.i < N - 1) {
+      const double jfac = P.fc.jdbl - j.d, ifac = P.fc.idbl - i.d;
+      const double accR = t00.x * (1 - ifac) * (1 - jfac) + t01.x * (1 - ifac) * jfac + t10.x * ifac * (1 - jfac) +
+                          t11.x * ifac * jfac;
+      const double accz = t00.y * (1 - ifac) * (1 - jfac) + t01.y * (1 - ifac) * jfac + t10.y * ifac * (1 - jfac) +
+                          t11.y * ifac * jfac;
+      P.a[0] = accR * cp;
+      P.a[1] = accR * sp;
+      P.a[2] = x[2] < 0 ? -accz : accz;
+    } else {
+      halo_acc(M, x, P.a);
+      const double fac = M.M200 / M.Halo_Mass;
+      for(int k = 0; k < 3; k++) P.a[k] *= fac;
+    }
+  } else
+    P.a[0] = P.a[1] = P.a[2] = 0;
+  if(M.analytic_halo) {
+    double h[3];
+    halo_acc(M, x, h);
+    for(int k = 0; k < 3; k++) P.a[k] += h[k];
+  }
+  if(M.analytic_bulge) {
+    double h[3];
+    bulge_acc(M, x, h);
+    for(int k = 0; k < 3; k++) P.a[k] += h[k];
+  }
+  return !step_ones(ones);
+}
+
+// What the end of a step gives: the projections, the next step's dt and the
+// radial sign's sum x.v
+struct Turn {
+  Proj proj;
+  double dt, radsign;
+};
+__device__ __noinline__ static Turn turn_general(const DevModel &M, Vec3 x, Vec3 v, Vec3 a, FgCoord fc, double Rxy,
+                                                 int icell, int type, int tovs, bool with_proj)
+{
+  Turn T{};
+  if(with_proj) T.proj = project(M, tovs, type, fc, x.c, v.c, Rxy);
+  T.dt = get_timestep(M, v.c, a.c, icell);
+  T.radsign = v.c[0] * x.c[0] + v.c[1] * x.c[1] + v.c[2] * x.c[2];
+  return T;
+}
+
+// the same for x (checked by place_fast) and v that step_safe accepts: the
+// products with the zero components of Z = (0, 0, -1) drop out (finite x; the
+// sign of a zero sum is lost in the squares), and the sums two expressions
+// share are formed once
+__device__ __forceinline__ bool turn_fast(const DevModel &M, const OrbitState &s, const Place &P, bool with_proj, Turn &T)
+{
+  const double *x = s.x, *v = s.v, *a = s.a;
+  const double cs = P.cs;
+  const double a2 = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+  if(!step_safe(v) || !step_safe_wide(a2) || !step_safe_wide(cs)) return false;
+  // get_timestep (orbit_response.c:16-26)
+  unsigned ones = 0;
+  const double vv = step_sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+  const double t1 = M.f_orb * step_div(M.V200, step_sqrt(a2), ones), t2 = M.f_cc * step_div(cs, vv, ones);
+  T.dt = t1 < t2 ? t1 : t2;
+  const double v_dot_x = v[0] * x[0] + v[1] * x[1] + v[2] * x[2];
+  T.radsign = v_dot_x;
+  if(with_proj) {
+    const double R2 = x[0] * x[0] + x[1] * x[1];
+    const double vq = step_div(v[1] * x[0] - v[0] * x[1], P.Rxy, ones);
+    const double vstr = vstream_at(M, P.fc, s.type);
+    T.proj.vq2 = vq * vq;
+    T.proj.vp2 = (vq - vstr) * (vq - vstr);
+    if(s.tovs == 2) {
+      const double vR = v[0] * x[0] + v[1] * x[1];
+      T.proj.vr2 = step_div(vR * vR, R2, ones);
+      T.proj.vt2 = v[2] * v[2];
+    } else {
+      T.proj.vr2 = step_div(v_dot_x * v_dot_x, R2 + x[2] * x[2], ones);
+      const double T0 = x[2] * x[0], T1 = x[2] * x[1];
+      const double v_dot_T = v[2] * R2 - (v[0] * T0 + v[1] * T1);
+      T.proj.vt2 = step_div(v_dot_T * v_dot_T, T0 * T0 + T1 * T1 + R2 * R2, ones);
+    }
+  }
+  return !step_ones(ones);
 }
 
 // One iteration of the do-loop of orbit_response.c:211-458 (with_proj) or
-// orbit_response.c:61-126 (mass only).  Calls sink(deposit) twice.  Returns
-// false when the orbit has ended.
+// orbit_response.c:61-126 (mass only), from the kick to the next iteration's
+// first half deposit: the end of one step and the start of the next are at
+// the same point, so both deposits go to one cell with one set of
+// projections (in the reference's order), and the sink changes cell at most
+// once per call.  Returns false when the orbit has ended.
 template <class Sink>
 __device__ __forceinline__ bool orbit_step(const DevModel &M, const LogConsts &L, OrbitState &s, bool with_proj,
                                            Sink &sink)
 {
-  const int Nb = M.DG_Nbin;
-  double dt = get_timestep(M, s.v, s.a, s.cell.iz * Nb + s.cell.iR);
-  if(0 < s.timespan)
-    if(s.timespan < dt + s.tall) {
-      dt = s.timespan - s.tall;
-      s.flag = 1;
-    }
-  sink(make_deposit(dt, s.cell, s.proj));
+  const double dt = s.dt;
   for(int i = 0; i < 3; i++) s.v[i] += 0.5 * dt * s.a[i];
   for(int i = 0; i < 3; i++) s.x[i] += dt * s.v[i];
-  // the four log coordinates of the new position (force grid: grid.c:130-136;
-  // density grid: grid.c:494-534) in one block, so that their independent
-  // chains interleave; the same expressions as fg_coord and density_cell
-  const double Rxy = sqrt(s.x[0] * s.x[0] + s.x[1] * s.x[1]), az = gm_fabs(s.x[2]);
-  const double lf0 = gm_log(div_by(Rxy, M.FG_Rmin, M.inv_FG_Rmin) + 1.0);
-  const double lf1 = gm_log(div_by(az, M.FG_Rmin, M.inv_FG_Rmin) + 1.0);
-  const double ld0 = gm_log(div_by(Rxy, M.DG_Rmin, M.inv_DG_Rmin) + 1.0);
-  const double ld1 = gm_log(div_by(az, M.DG_Rmin, M.inv_DG_Rmin) + 1.0);
-  FgCoord fc;
-  fc.jdbl = div_by(lf0, L.lfg, M.inv_lfg);
-  fc.idbl = div_by(lf1, L.lfg, M.inv_lfg);
-  forcegrid_acc(M, fc, s.x, s.a);
+  Place P;
+  const bool fast = place_fast(M, L, s.x, P);
+  if(!fast) P = place_general(M, {s.x[0], s.x[1], s.x[2]});
+  for(int i = 0; i < 3; i++) s.a[i] = P.a[i];
   for(int i = 0; i < 3; i++) s.v[i] += 0.5 * dt * s.a[i];
-  s.cell = cell_from_b(div_by(ld0, L.ldg, M.inv_ldg) - 0.5, div_by(ld1, L.ldg, M.inv_ldg) - 0.5, M.DG_Nbin);
-  if(with_proj) s.proj = project(M, s.tovs, s.type, fc, s.x, s.v, Rxy);
-  sink(make_deposit(dt, s.cell, s.proj));
+  sink.enter(P.cell.iR, P.cell.iz);
+  Turn T;
+  if(!fast || !turn_fast(M, s, P, with_proj, T))
+    T = turn_general(M, {s.x[0], s.x[1], s.x[2]}, {s.v[0], s.v[1], s.v[2]}, {s.a[0], s.a[1], s.a[2]}, P.fc, P.Rxy,
+                     P.cell.iz * M.DG_Nbin + P.cell.iR, s.type, s.tovs, with_proj);
   s.tall += dt;
-  double radsign = s.v[0] * s.x[0] + s.v[1] * s.x[1] + s.v[2] * s.x[2];
-  if(radsign > 0 && s.rad_in) s.norbit++;
-  s.rad_in = radsign < 0;
+  if(T.radsign > 0 && s.rad_in) s.norbit++;
+  s.rad_in = T.radsign < 0;
   s.steps++;
-  if(!(s.tall == s.tall) || !(dt == dt)) {
-    s.status = ORBIT_NONFINITE;
-    return false;
-  }
-  if(s.steps > M.step_cap) {
-    s.status = ORBIT_STEP_CAP;
-    return false;
-  }
   // (timespan == 0 && norbit < Norbits) continues until the step cap, as in
   // the reference (Norbits = 1e8)
-  return (s.timespan == 0 && s.norbit < 100000000) || (s.timespan != 0 && s.flag == 0);
+  bool more = (s.timespan == 0 && s.norbit < 100000000) || (s.timespan != 0 && s.flag == 0);
+  if(s.steps > M.step_cap) {
+    s.status = ORBIT_STEP_CAP;
+    more = false;
+  }
+  if(!(s.tall == s.tall) || !(dt == dt)) {
+    s.status = ORBIT_NONFINITE;
+    more = false;
+  }
+  if(more) set_step(s, T.dt);
+  sink.add(P.cell, 0.5 * dt, more ? 0.5 * s.dt : 0.0, T.proj);
+  return more;
 }
 
 // orbit_response.c:460-462: relative energy error of the finished orbit

@@ -92,25 +92,33 @@ struct ParkSink {
     parked = true;
     cur = -1;
   }
-  __device__ __forceinline__ void operator()(const Deposit &d)
+  __device__ __forceinline__ void enter(int iR, int iz)
   {
-    int c = d.iz * Nb + d.iR;
-    if(c != cur) {
-      park();
+    const int c = iz * Nb + iR;
+    if(c == cur) return;
+    park();
 #pragma unroll
-      for(int k = 0; k < 4; k++)
+    for(int k = 0; k < 4; k++)
 #pragma unroll
-        for(int f = 0; f < 5; f++) a[k][f] = 0;
-      cur = c;
-    }
-    const double w[4] = {d.m00, d.m10, d.m01, d.m11};
+      for(int f = 0; f < 5; f++) a[k][f] = 0;
+    cur = c;
+  }
+  __device__ __forceinline__ void add(const Cell &k, double hdt, double next_hdt, const Proj &p)
+  {
+    add_one(k, hdt, p);
+    add_one(k, next_hdt, p);
+  }
+  __device__ __forceinline__ void add_one(const Cell &k, double hdt, const Proj &p)
+  {
+    const double w[4] = {hdt * (1 - k.fR) * (1 - k.fz), hdt * (k.fR) * (1 - k.fz), hdt * (1 - k.fR) * (k.fz),
+                         hdt * (k.fR) * (k.fz)};
 #pragma unroll
-    for(int k = 0; k < 4; k++) {
-      a[k][0] += w[k];
-      a[k][1] += w[k] * d.p.vr2;
-      a[k][2] += w[k] * d.p.vt2;
-      a[k][3] += w[k] * d.p.vq2;
-      a[k][4] += w[k] * d.p.vp2;
+    for(int c = 0; c < 4; c++) {
+      a[c][0] += w[c];
+      a[c][1] += w[c] * p.vr2;
+      a[c][2] += w[c] * p.vt2;
+      a[c][3] += w[c] * p.vq2;
+      a[c][4] += w[c] * p.vp2;
     }
   }
 };
@@ -135,7 +143,7 @@ __device__ __forceinline__ void drain(Slots &q, unsigned full, const NoAllocArgs
 
 enum { ST_ACTIVE = 0, ST_FINISH = 1, ST_DONE = 2 };
 
-__global__ void __launch_bounds__(128, 3) k_noalloc_orbits(DevModel M, NoAllocArgs A)
+__global__ void __launch_bounds__(128, 3) k_noalloc_orbits(const __grid_constant__ DevModel M, NoAllocArgs A)
 {
   __shared__ Slots queues[4];
   LogConsts L = step_log_consts(M);
@@ -167,7 +175,7 @@ __global__ void __launch_bounds__(128, 3) k_noalloc_orbits(DevModel M, NoAllocAr
     sink.type = A.type[p];
     sink.fac = A.mass[p] / A.tint[p];
     sink.cur = -1;
-    orbit_begin(M, L, s, &A.pos[3 * p], &A.vel[3 * p], A.tint[p], sink.type, true);
+    orbit_begin(M, L, s, &A.pos[3 * p], &A.vel[3 * p], A.tint[p], sink.type, true, sink);
     return true;
   };
   int state = fetch() ? ST_ACTIVE : ST_DONE;

@@ -598,7 +598,7 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
     // records carry the orbit's grid set and scale only through the lane's
     // queue header, so a lane drains them before it starts the next orbit
     if(queue32_due<PER>(sink.cnt) || __any_sync(0xffffffffu, (all_done || state == LANE_START) && sink.cnt > 0))
-      warp_drain32(*sink.q, (FxNode32 *) S.fx, sink.cnt);
+      warp_drain_nodes(*sink.q, (FxNode *) S.fx, sink.cnt);
     if(all_done) break;
     if(state == LANE_ACTIVE) {
       if(!orbit32_step<Sink32<PER>, true>(S.model(mi), s, sink)) state = s.status == ORBIT_OK ? LANE_LAST : LANE_FINISH;

@@ -19,87 +19,122 @@
 
 namespace {
 
+// The four nodes of a cell by parity: node (z, r) lives in slot
+// ((z & 1) << 1) | (r & 1), so that when an orbit moves to a neighbouring cell
+// the nodes the two cells share keep their slots.
+struct SlotNodes {
+  int z[2], r[2];  // the even and the odd node along each axis
+  __device__ __forceinline__ SlotNodes() : z{-1, -1}, r{-1, -1} {}
+  __device__ __forceinline__ SlotNodes(int iR, int iz) : z{(iz + 1) & ~1, iz | 1}, r{(iR + 1) & ~1, iR | 1} {}
+  __device__ __forceinline__ int index(int slot, int Nb) const { return z[slot >> 1] * Nb + r[slot & 1]; }
+  // out[slot]: the slot's node is not one of `next`
+  __device__ __forceinline__ void leaving(const SlotNodes &next, bool out[4]) const
+  {
+    const bool lz[2] = {z[0] != next.z[0], z[1] != next.z[1]}, lr[2] = {r[0] != next.r[0], r[1] != next.r[1]};
+#pragma unroll
+    for(int k = 0; k < 4; k++) out[k] = lz[k >> 1] || lr[k & 1];
+  }
+};
+// the weights of a half step for cell c's nodes in slot order (products in
+// the order of orbit_response.c:277-320)
+__device__ __forceinline__ void slot_weights(const Cell &c, double hdt, double w[4])
+{
+  const bool oz = c.iz & 1, orr = c.iR & 1;
+  const double z0 = oz ? c.fz : 1 - c.fz, z1 = oz ? 1 - c.fz : c.fz;
+  const double r0 = orr ? c.fR : 1 - c.fR, r1 = orr ? 1 - c.fR : c.fR;
+  w[0] = hdt * r0 * z0;
+  w[1] = hdt * r1 * z0;
+  w[2] = hdt * r0 * z1;
+  w[3] = hdt * r1 * z1;
+}
+
+// The orbit's own dense grids [NF_ORBIT][G] in global memory.  The bins of
+// the cell the orbit is in are held in registers, by slot: a deposit adds to
+// them in the reference's order per bin (bin += value); when the orbit moves
+// to another cell, enter() stores the bins whose node leaves and loads those
+// of the nodes that come in, and finish() stores the last cell's.  Each
+// orbit's grids are its own, so every bin receives the reference's sequence of
+// roundings.  enter() is called before the step's projections, so that they
+// cover the loads.
 struct DenseSink {
-  double *m, *r, *t, *q, *p;
-  int Nb;
+  double *grid;
+  int G, Nb;
   int with_egy;
-  // The bins of the cell the orbit is in, held in registers: c[f][corner]
-  // for corners 00, 10, 01, 11.  A deposit adds to them in the reference's
-  // order per bin (bin += value); when a deposit falls in another cell the
-  // held bins are stored and the new cell's bins loaded (a bin two cells
-  // share is stored before it is loaded again), and finish() stores the
-  // last cell's.  Each orbit's grids are its own, so every bin receives the
-  // reference's sequence of roundings, and the thread waits for the grid
-  // only when the orbit changes cell instead of at every deposit.
-  int cur = -1;  // grid index of the held cell's corner 00; -1: none
-  double c[5][4];
-  __device__ __forceinline__ double *field(int f) const
+  bool held = false;
+  SlotNodes node;  // the held cell's nodes
+  double c[4][5];
+  __device__ __forceinline__ void store_slots(const bool which[4])
   {
-    return f == 0 ? m : f == 1 ? r : f == 2 ? t : f == 3 ? q : p;
-  }
-  __device__ __forceinline__ void store_cell()
-  {
-    const int idx[4] = {cur, cur + 1, cur + Nb, cur + Nb + 1};
-    const int nf = with_egy ? 5 : 1;
 #pragma unroll
-    for(int f = 0; f < 5; f++)
-      if(f < nf) {
-        double *g = field(f);
-#pragma unroll
-        for(int k = 0; k < 4; k++) g[idx[k]] = c[f][k];
+    for(int k = 0; k < 4; k++) {
+      if(!which[k]) continue;
+      double *g = grid + node.index(k, Nb);
+      g[F_M * G] = c[k][0];
+      if(with_egy) {
+        g[F_R * G] = c[k][1];
+        g[F_T * G] = c[k][2];
+        g[F_Q * G] = c[k][3];
+        g[F_P * G] = c[k][4];
       }
-  }
-  __device__ __forceinline__ void load_cell(int i00)
-  {
-    const int idx[4] = {i00, i00 + 1, i00 + Nb, i00 + Nb + 1};
-    const int nf = with_egy ? 5 : 1;
-#pragma unroll
-    for(int f = 0; f < 5; f++)
-      if(f < nf) {
-        const double *g = field(f);
-#pragma unroll
-        for(int k = 0; k < 4; k++) c[f][k] = g[idx[k]];
-      }
-    cur = i00;
-  }
-  __device__ __forceinline__ void operator()(const Deposit &d)
-  {
-    const int i00 = d.iz * Nb + d.iR;
-    if(i00 != cur) {
-      if(cur >= 0) store_cell();
-      load_cell(i00);
     }
-    const double w[4] = {d.m00, d.m10, d.m01, d.m11};
+  }
+  __device__ __forceinline__ void enter(int iR, int iz)
+  {
+    const SlotNodes next(iR, iz);
+    bool out[4];
+    node.leaving(next, out);
+    if(held) store_slots(out);
+    held = true;
+    node = next;
 #pragma unroll
-    for(int k = 0; k < 4; k++) c[0][k] = c[0][k] + w[k];
-    if(with_egy) {
+    for(int k = 0; k < 4; k++) {
+      if(!out[k]) continue;
+      const double *g = grid + node.index(k, Nb);
+      c[k][0] = g[F_M * G];
+      if(with_egy) {
+        c[k][1] = g[F_R * G];
+        c[k][2] = g[F_T * G];
+        c[k][3] = g[F_Q * G];
+        c[k][4] = g[F_P * G];
+      }
+    }
+  }
+  __device__ __forceinline__ void add(const Cell &cell, double hdt, double next_hdt, const Proj &p)
+  {
+    double w[4], n[4];
+    slot_weights(cell, hdt, w);
+    slot_weights(cell, next_hdt, n);
 #pragma unroll
-      for(int k = 0; k < 4; k++) {
-        c[1][k] = c[1][k] + w[k] * d.p.vr2;
-        c[2][k] = c[2][k] + w[k] * d.p.vt2;
-        c[3][k] = c[3][k] + w[k] * d.p.vq2;
-        c[4][k] = c[4][k] + w[k] * d.p.vp2;
+    for(int k = 0; k < 4; k++) {
+      c[k][0] = c[k][0] + w[k] + n[k];
+      if(with_egy) {
+        c[k][1] = c[k][1] + w[k] * p.vr2 + n[k] * p.vr2;
+        c[k][2] = c[k][2] + w[k] * p.vt2 + n[k] * p.vt2;
+        c[k][3] = c[k][3] + w[k] * p.vq2 + n[k] * p.vq2;
+        c[k][4] = c[k][4] + w[k] * p.vp2 + n[k] * p.vp2;
       }
     }
   }
   __device__ __forceinline__ void finish()
   {
-    if(cur >= 0) store_cell();
-    cur = -1;
+    const bool all[4] = {true, true, true, true};
+    if(held) store_slots(all);
   }
 };
 
-__global__ void k_orbits_dense(DevModel M, OrbitBatch b)
+__global__ void k_orbits_dense(const __grid_constant__ DevModel M, OrbitBatch b)
 {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if(k >= b.count) return;
   LogConsts L = step_log_consts(M);
   const size_t G = (size_t) M.DG_Ngrid;
-  double *base = b.grids + (size_t) k * NF_ORBIT * G;
-  DenseSink sink{base + F_M * G, base + F_R * G, base + F_T * G, base + F_Q * G, base + F_P * G, M.DG_Nbin,
-                 b.with_egy};
+  DenseSink sink;
+  sink.grid = b.grids + (size_t) k * NF_ORBIT * G;
+  sink.G = (int) G;
+  sink.Nb = M.DG_Nbin;
+  sink.with_egy = b.with_egy;
   OrbitState s;
-  orbit_begin(M, L, s, &b.pos[3 * k], &b.vel[3 * k], b.timespan[k], b.type[k], b.with_egy != 0);
+  orbit_begin(M, L, s, &b.pos[3 * k], &b.vel[3 * k], b.timespan[k], b.type[k], b.with_egy != 0, sink);
   while(orbit_step(M, L, s, b.with_egy != 0, sink)) {
   }
   sink.finish();
@@ -125,20 +160,17 @@ __global__ void k_scale_dense(OrbitBatch b, int G)
 }
 
 // Node sink of the batched path.  The deposits of consecutive steps are
-// summed per grid NODE in FP64 registers: node (z, r) lives in accumulator
-// slot ((z & 1) << 1) | (r & 1), so the four nodes of any cell have the four
-// parities, and when the orbit moves to a neighbouring cell the nodes the two
-// cells share stay in place.  Only the slots whose node leaves are parked, as
-// records {node index, 5 sums}, in the lane's column of the warp's queue; the
-// warp drains all lanes' records together (flush.cuh:warp_drain64),
-// each value scaled by mass/Tint and added as an exact two-word fixed-point
-// pair (order independent).
+// summed per grid NODE in FP64 registers, by slot (see SlotNodes).  Only the
+// slots whose node leaves are parked, as records {node index, 5 sums}, in the
+// lane's column of the warp's queue; the warp drains all lanes' records
+// together (flush.cuh:warp_drain_nodes), each value scaled by mass/Tint and added
+// as an exact two-word fixed-point pair (order independent).
 template <int PER>
 struct NodeSink64 {
   WarpQueue64<PER> *q;
   int lane, Nb;
   int cnt;  // records parked in this lane's column since the last drain
-  int cur_iR, cur_iz;  // the current cell; cur_iz < 0: none
+  SlotNodes node;  // the current cell's nodes
   double a[4][5];
   // fac x 2^(shift - 24) of the mass and the energy fields (exact scalings)
   __device__ __forceinline__ void set_orbit(int gbase, double scale_m, double scale_e)
@@ -146,82 +178,60 @@ struct NodeSink64 {
     q->gbase[lane] = gbase;
     q->scale[0][lane] = scale_m;
     q->scale[1][lane] = scale_e;
-    cur_iz = -1;
-  }
-  // slot s of cell (iz, iR) holds node (iz + node_dz(s, iz), iR + node_dr(s, iR))
-  __device__ __forceinline__ static int node_dz(int s, int iz) { return ((s >> 1) ^ iz) & 1; }
-  __device__ __forceinline__ static int node_dr(int s, int iR) { return (s ^ iR) & 1; }
-  __device__ __forceinline__ void park_masked(const bool out[4])
-  {
-    // record positions first, then predicated stores: straight-line code
-    // for every lane of the warp
-    bool rec[4];
-    int at[4], k = cnt;
-#pragma unroll
-    for(int s = 0; s < 4; s++) {
-      rec[s] = out[s] && a[s][0] != 0.0;  // a node without mass has no deposit at all
-      at[s] = k;
-      k += rec[s] ? 1 : 0;
-    }
-#pragma unroll
-    for(int s = 0; s < 4; s++) {
-      if(rec[s]) {
-        q->base[at[s]][lane] = (cur_iz + node_dz(s, cur_iz)) * Nb + cur_iR + node_dr(s, cur_iR);
-#pragma unroll
-        for(int f = 0; f < 5; f++) q->val[at[s]][f][lane] = a[s][f];
-      }
-    }
-    cnt = k;
-  }
-  __device__ __forceinline__ void park()
-  {
-    if(cur_iz < 0) return;
-    const bool all[4] = {true, true, true, true};
-    park_masked(all);
-    cur_iz = -1;
-  }
-  __device__ __forceinline__ void move_to(int iR, int iz)
-  {
-    bool out[4];
-    if(cur_iz >= 0) {
-      // along one axis a move by d leaves the node whose parity is that of
-      // the boundary left behind, both nodes when |d| > 1, none when d = 0
-      const int dz = iz - cur_iz, dr = iR - cur_iR;
-      const int bz = (dz > 0 ? cur_iz : cur_iz + 1) & 1, br = (dr > 0 ? cur_iR : cur_iR + 1) & 1;
-      const bool zall = dz > 1 || dz < -1, rall = dr > 1 || dr < -1;
-#pragma unroll
-      for(int s = 0; s < 4; s++)
-        out[s] = (zall || (dz != 0 && (s >> 1) == bz)) || (rall || (dr != 0 && (s & 1) == br));
-      park_masked(out);
-    } else {
-#pragma unroll
-      for(int s = 0; s < 4; s++) out[s] = true;
-    }
 #pragma unroll
     for(int s = 0; s < 4; s++)
 #pragma unroll
-      for(int f = 0; f < 5; f++) a[s][f] = out[s] ? 0.0 : a[s][f];
-    cur_iR = iR;
-    cur_iz = iz;
+      for(int f = 0; f < 5; f++) a[s][f] = 0.0;
   }
-  __device__ __forceinline__ void operator()(const Deposit &d)
+  // parks the slots in out that hold a deposit (a node without mass has none)
+  __device__ __forceinline__ void park_masked(const bool out[4])
   {
-    if(d.iz != cur_iz || d.iR != cur_iR) move_to(d.iR, d.iz);
-    // slot s holds corner (dz, dr) = ((s >> 1) ^ (iz & 1), (s & 1) ^ (iR & 1));
-    // corner weights: (0,0) m00, (0,1) m10, (1,0) m01, (1,1) m11
-    const bool oz = d.iz & 1, orr = d.iR & 1;
-    const double z0r0 = oz ? d.m01 : d.m00, z0r1 = oz ? d.m11 : d.m10;  // slot z-parity 0: dz = oz
-    const double z1r0 = oz ? d.m00 : d.m01, z1r1 = oz ? d.m10 : d.m11;
-    const double w[4] = {orr ? z0r1 : z0r0, orr ? z0r0 : z0r1, orr ? z1r1 : z1r0, orr ? z1r0 : z1r1};
-    // the node sums are this form's own partial sums (the reference adds
-    // every product to the grid bin in turn): fused, one rounding per term
+    // straight-line code for every lane of the warp: some lane of 32 changes
+    // cell on nearly every step
+#pragma unroll
+    for(int s = 0; s < 4; s++) {
+      if(out[s] && a[s][0] != 0.0) {
+        q->base[cnt][lane] = (unsigned short) node.index(s, Nb);
+#pragma unroll
+        for(int f = 0; f < 5; f++) q->val[cnt][f][lane] = a[s][f];
+        cnt++;
+      }
+    }
+  }
+  __device__ __forceinline__ void park()
+  {
+    const bool all[4] = {true, true, true, true};
+    park_masked(all);
+  }
+  __device__ __forceinline__ void enter(int iR, int iz)
+  {
+    const SlotNodes next(iR, iz);
+    if(next.z[0] == node.z[0] && next.z[1] == node.z[1] && next.r[0] == node.r[0] && next.r[1] == node.r[1]) return;
+    bool out[4];
+    node.leaving(next, out);
+    park_masked(out);
+#pragma unroll
+    for(int s = 0; s < 4; s++)
+      if(out[s]) {
+#pragma unroll
+        for(int f = 0; f < 5; f++) a[s][f] = 0.0;
+      }
+    node = next;
+  }
+  // the node sums are this form's own partial sums (the reference adds
+  // every product to the grid bin in turn): fused, one rounding per term
+  __device__ __forceinline__ void add(const Cell &cell, double hdt, double next_hdt, const Proj &p)
+  {
+    double w[4], n[4];
+    slot_weights(cell, hdt, w);
+    slot_weights(cell, next_hdt, n);
 #pragma unroll
     for(int k = 0; k < 4; k++) {
-      a[k][0] += w[k];
-      a[k][1] = fma(w[k], d.p.vr2, a[k][1]);
-      a[k][2] = fma(w[k], d.p.vt2, a[k][2]);
-      a[k][3] = fma(w[k], d.p.vq2, a[k][3]);
-      a[k][4] = fma(w[k], d.p.vp2, a[k][4]);
+      a[k][0] = a[k][0] + w[k] + n[k];
+      a[k][1] = fma(n[k], p.vr2, fma(w[k], p.vr2, a[k][1]));
+      a[k][2] = fma(n[k], p.vt2, fma(w[k], p.vt2, a[k][2]));
+      a[k][3] = fma(n[k], p.vq2, fma(w[k], p.vq2, a[k][3]));
+      a[k][4] = fma(n[k], p.vp2, fma(w[k], p.vp2, a[k][4]));
     }
   }
 };
@@ -239,7 +249,7 @@ enum LaneState { LANE_ACTIVE = 0, LANE_FINISH = 1, LANE_DONE = 2, LANE_START = 3
 constexpr int kPer64 = 8;
 
 template <int MINB>
-__global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(DevModel M, CalcAllArgs A)
+__global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(const __grid_constant__ DevModel M, CalcAllArgs A)
 {
   __shared__ WarpQueue64<kPer64> queues[CALC_ALL_BLOCK_FP64 / 32];
   // the CTA's step count, largest energy error (as bits: non-negative
@@ -260,7 +270,6 @@ __global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(Dev
   sink.q = &queues[threadIdx.x >> 5];
   sink.lane = threadIdx.x & 31;
   sink.Nb = M.DG_Nbin;
-  sink.cur_iz = -1;
   sink.cnt = 0;
   int p = -1;
 
@@ -275,9 +284,9 @@ __global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(Dev
     p = A.order ? A.order[k] : k;
     const int type = A.type[p];
     const double fac = A.mass[p] / A.tint[p];
-    sink.set_orbit(type * NG_COMMITTED * G, ldexp(fac, A.shift[type * NG_COMMITTED + GALIC_GRID_MASS_S] - 24),
+    sink.set_orbit(2 * type * G, ldexp(fac, A.shift[type * NG_COMMITTED + GALIC_GRID_MASS_S] - 24),
                    ldexp(fac, A.shift[type * NG_COMMITTED + GALIC_GRID_R_S] - 24));
-    orbit_begin(M, L, s, &A.pos[3 * p], &A.vel[3 * p], A.tint[p], type, true);
+    orbit_begin(M, L, s, &A.pos[3 * p], &A.vel[3 * p], A.tint[p], type, true, sink);
     return true;
   };
 
@@ -288,7 +297,7 @@ __global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(Dev
     // header: a lane's records are drained before it starts the next orbit
     if(queue32_due<kPer64>(sink.cnt) ||
        __any_sync(0xffffffffu, (all_done || state == LANE_START) && sink.cnt > 0))
-      warp_drain64(*sink.q, A.fx, G, sink.cnt);
+      warp_drain_nodes(*sink.q, (FxNode *) A.fx, sink.cnt);
     if(all_done) break;
     if(state == LANE_ACTIVE) {
       if(!orbit_step(M, L, s, true, sink)) state = LANE_FINISH;
@@ -346,19 +355,21 @@ __global__ void k_instantaneous(DevModel M, int n, int first, int stride, const 
   }
 }
 
-// fp32: the time-averaged grids of every set hold its FxNode32 words
-__global__ void k_fx_finalize(const FxWord *fx, const int *shift, double *out, int count, int Ngrid, bool fp32)
+// The time-averaged half of every set holds FxNode words (one_word: the FP32
+// form's single words), the instantaneous half word pairs grid by grid.
+__global__ void k_fx_finalize(const FxWord *fx, const int *shift, double *out, int count, int Ngrid, bool one_word)
 {
   size_t total = (size_t) count * Ngrid;
   for(size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < total; i += (size_t) gridDim.x * blockDim.x) {
-    int g = (int) (i / Ngrid);
-    FxWord w = fx[i];
-    if(fp32 && g % NG_COMMITTED < NF_ORBIT) {
-      // the first five grids of a set are half of its NG_COMMITTED
-      const FxNode32 *nodes = (const FxNode32 *) fx + (size_t) (g / NG_COMMITTED) * 2 * Ngrid;
-      w.hi = nodes[i % Ngrid].w[g % NG_COMMITTED];
-      w.lo = 0;
-    }
+    const int g = (int) (i / Ngrid), f = g % NG_COMMITTED;
+    FxWord w;
+    if(f < NF_ORBIT) {
+      // (a set's first five grids are half of its NG_COMMITTED)
+      const FxNode *n = (const FxNode *) fx + (size_t) (g / NG_COMMITTED) * 2 * Ngrid + i % Ngrid;
+      w.hi = n->hi[f];
+      w.lo = one_word ? 0 : n->lo[f];
+    } else
+      w = fx[i];
     out[i] = fx_value(w, shift[g]);
   }
 }

@@ -1,0 +1,132 @@
+"""The orbit step's branch-free arithmetic (galic_b200/csrc/stepmath.cuh) equals the general functions bit for bit.
+
+The kernels take it for operands in its stated ranges and the general
+functions otherwise; the per-orbit parity tests cover whole orbits, these the
+functions themselves (random operands, quotients and roots next to rounding
+boundaries, table and octant edges) and orbits whose operands leave the ranges."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from galic_b200 import Context, synth
+from oracle_lib import Oracle
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SRC = r'''
+#include "gmath.h"
+#include "stepmath.cuh"
+__global__ void k_cmp(int n, const double *a, const double *b, int what, unsigned *bad)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if(i >= n) return;
+  const double x = a[i], y = b[i];
+  bool ok = true;
+  unsigned ones = 0;  // operands the functions refuse
+  if(what == 0) ok = step_div(x, y, ones) == x / y || step_ones(ones);
+  if(what == 1) ok = step_sqrt(x) == sqrt(x);
+  if(what == 2) ok = step_log(x) == gm_log(x);
+  if(what == 3) {
+    double s, c, s0, c0;
+    step_direction(x, y, &s, &c, ones);
+    gm_sincos(gm_atan2(x, y), &s0, &c0);
+    ok = (s == s0 && c == c0) || step_ones(ones);
+  }
+  if(what == 4) {
+    const StepFloor f = step_floor(x);
+    ok = f.i == (int) x && f.d == (double) (int) x;
+  }
+  if(!ok) atomicAdd(bad, 1u);
+}
+extern "C" int compare(int n, const double *a, const double *b, int what)
+{
+  double *da, *db;
+  unsigned *bad, h = 0;
+  if(cudaMalloc(&da, n * 8) || cudaMalloc(&db, n * 8) || cudaMalloc(&bad, 4)) return -1;
+  cudaMemcpy(da, a, n * 8, cudaMemcpyHostToDevice);
+  cudaMemcpy(db, b, n * 8, cudaMemcpyHostToDevice);
+  cudaMemset(bad, 0, 4);
+  k_cmp<<<(n + 255) / 256, 256>>>(n, da, db, what, bad);
+  if(cudaMemcpy(&h, bad, 4, cudaMemcpyDeviceToHost)) return -1;
+  cudaFree(da); cudaFree(db); cudaFree(bad);
+  return (int) h;
+}
+'''
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("step")
+    (d / "t.cu").write_text(SRC)
+    subprocess.run(["/usr/local/cuda/bin/nvcc", "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "--fmad=false", "-shared", "-Xcompiler", "-fPIC", "-I", os.path.join(ROOT, "galic_b200", "csrc"),
+                    str(d / "t.cu"), "-o", str(d / "libt.so")], check=True)
+    return C.CDLL(str(d / "libt.so"))
+
+
+def _significands(rng, n):
+    """Random significands in [1, 2), a quarter of them next to 1 or 2."""
+    m = 1.0 + rng.integers(0, 1 << 52, n) * 2.0 ** -52
+    k = n // 8
+    m[:k] = 1.0 + rng.integers(0, 16, k) * 2.0 ** -52
+    m[k:2 * k] = 2.0 - (1 + rng.integers(0, 16, k)) * 2.0 ** -52
+    return rng.permutation(m)
+
+
+def _operands(what, rng, n):
+    scale = np.ldexp(1.0, rng.integers(-100, 100, n))
+    a, b = _significands(rng, n) * scale, _significands(rng, n) * np.ldexp(1.0, rng.integers(-100, 100, n))
+    sign = rng.choice([-1.0, 1.0], n)
+    if what == 0:  # half of the quotients within a few ulp of a rounding boundary
+        q = _significands(rng, n)
+        near = np.asarray([float(x) for x in (b.astype(np.longdouble) * (q.astype(np.longdouble) + 2.0 ** -53))])
+        return np.where(rng.random(n) < 0.5, near * (1 + rng.integers(-2, 3, n) * 2.0 ** -52), a) * sign, b
+    if what == 1:
+        q = _significands(rng, n).astype(np.longdouble) + np.longdouble(2.0 ** -53)
+        near = (q * q).astype(np.float64) * (1 + rng.integers(-2, 3, n) * 2.0 ** -52)
+        return np.where(rng.random(n) < 0.5, near * np.ldexp(1.0, 2 * rng.integers(-50, 50, n)), a * a), b
+    if what == 2:  # table edges (1 + j / 128 and their midpoints) among them
+        edge = 1.0 + rng.integers(0, 512, n) / 256.0 * (1 + rng.integers(-2, 3, n) * 2.0 ** -52)
+        return np.maximum(np.where(rng.random(n) < 0.3, edge, _significands(rng, n) * np.ldexp(1.0, rng.integers(0, 300, n))), 1.0), b
+    if what == 3:  # all octants, ratios next to the table's k / 16 among them, tiny angles
+        ratio = rng.integers(1, 17, n) / 16.0 * (1 + rng.integers(-2, 3, n) * 2.0 ** -52)
+        x = b * rng.choice([-1.0, 1.0], n)
+        y = np.where(rng.random(n) < 0.5, np.abs(x) * ratio, np.abs(x) * np.exp(rng.uniform(-40, 40, n)))
+        y = np.clip(y, 2.0 ** -99, 2.0 ** 99) * sign
+        swap = rng.random(n) < 0.5
+        return np.where(swap, x, y), np.where(swap, y, x)
+    return rng.choice([0.0, 1.0], n) * rng.integers(0, 2 ** 31 - 1, n) + rng.choice([0.0, 0.5, 2.0 ** -52], n), b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", [0, 1, 2, 3, 4], ids=["div", "sqrt", "log", "direction", "floor"])
+def test_step_functions_equal_the_general_ones(lib, what):
+    a, b = _operands(what, np.random.default_rng(what), 4_000_000)
+    a, b = np.ascontiguousarray(a, dtype=np.float64), np.ascontiguousarray(b, dtype=np.float64)
+    P = C.POINTER(C.c_double)
+    assert lib.compare(len(a), a.ctypes.data_as(P), b.ctypes.data_as(P), what) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", ["halo", "halo_disk"])
+def test_orbits_outside_the_step_ranges_equal_the_oracle(shape):
+    """Planar, axial, cold and nearly planar orbits, one beyond the force grid: every bin, the time and the orbit count."""
+    m = synth.config_halo(n=32, level=5, seed=3) if shape == "halo" else synth.config_halo_disk(24, 8, level=5, seed=3)
+    o = Oracle(m.params, use_libm=False)
+    o.load_model(m)
+    x, v = m.pos[0], m.vel[0]
+    far = 3.0 * m.meta["rmax"] * x / np.linalg.norm(x)
+    starts = [(x * [1, 1, 0], v * [1, 1, 0]), (x * [0, 1, 1], v * [0, 1, 1]), (x, v * 0), (x * [1, 1, 1e-40], v * [1, 1, 0]),
+              (x * [1, 1e-35, 1], v * [1, 1e-200, 1]), (far, v)]
+    with Context(m.params) as ctx:
+        ctx.load_model(m)
+        for t in {int(k) for k in m.ptype}:
+            for p, w in starts:
+                got = ctx.produce_orbit_response_field_mod(p, w, m.mass[0], m.tint[0], t)
+                want = o.orbit_mod(np.ascontiguousarray(p), np.ascontiguousarray(w), m.mass[0], m.tint[0], t)
+                assert got[0] == want[0] and got[1] == want[1]
+                for a, b in zip(got[2:], want[2:7]):
+                    assert np.array_equal(a, b, equal_nan=True)
