@@ -609,6 +609,16 @@ namespace galic_internal {
 
 cudaError_t keep_device_pool(int device) { return keep_pool_memory(device); }
 
+cudaError_t second_stream(galic_ctx *ctx)
+{
+  cudaError_t e = cudaSuccess;
+  for(int k = 0; k < 5 && e == cudaSuccess; k++)
+    if(!ctx->ev2[k]) e = cudaEventCreateWithFlags(&ctx->ev2[k], cudaEventDisableTiming);
+  if(e == cudaSuccess && !ctx->stream2)
+    e = cudaStreamCreateWithPriority(&ctx->stream2, cudaStreamNonBlocking, ctx->priority);
+  return e;
+}
+
 // installs particles whose arrays are on the device, stored type by type
 // (nt[t] particles of type t, masses tmass[t] / nt[t]), as galic_set_particles
 // does from the host
@@ -1211,10 +1221,7 @@ extern "C" int galic_optimize_reps(galic_ctx *ctx, const int *idx, int count, in
     CK(dalloc(ctx, &ctx->d_idx_all, (size_t) reps * count));
     ctx->idx_cap = (size_t) reps * count;
   }
-  if(!ctx->stream2) {
-    CK(cudaStreamCreateWithPriority(&ctx->stream2, cudaStreamNonBlocking, ctx->priority));
-    for(int k = 0; k < 5; k++) CK(cudaEventCreateWithFlags(&ctx->ev2[k], cudaEventDisableTiming));
-  }
+  CK(second_stream(ctx));
   cudaStream_t so = ctx->stream2;
   // every index of the call in one copy; staged through pinned memory
   {

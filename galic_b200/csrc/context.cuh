@@ -108,6 +108,8 @@ int ensure_tab32(galic_ctx *ctx);
 FitArgs make_fit_args(galic_ctx *ctx);
 // keeps the device's default memory pool mapped between calls (once per device)
 cudaError_t keep_device_pool(int device);
+// creates the context's second stream (stream2) and its events (ev2) once
+cudaError_t second_stream(galic_ctx *ctx);
 // installs particles whose arrays are on the device, stored type by type
 int set_particles_device(galic_ctx *ctx, const int nt[4], const double tmass[4], const double *pos,
                          const double *vel, const double *tint, const double *vesc, const double *targets);

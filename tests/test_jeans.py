@@ -136,3 +136,16 @@ def test_gpu_tables_feed_the_context():
         with pytest.raises(GalicError) as e:  # the reference's terminate()
             jeans.calculate_dispfield(ctx, sp, bad)
         assert e.value.status == 6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fg_nbin", [3, 22, 23, 264, 265, 529])
+def test_gpu_tilted_march_column_counts(fg_nbin):
+    """One warp's columns and one more, the largest counts of the march's CTA sizes and one more."""
+    m = jeans_model(fg_nbin=fg_nbin, tovs=(0, 3, 0))
+    sp, jp = jeans_params(m, 0.0, 0.0)
+    got, _ = _gpu_dispfield(m, sp, jp)
+    st, ref = oracle_lib.oracle_dispfield(m, sp, jp, use_libm=False)
+    assert st == 0
+    for w, name in enumerate(_ffi.JEANS_TABLES):
+        assert np.array_equal(got[2][name], ref[2, w], equal_nan=True), name
