@@ -489,7 +489,7 @@ extern "C" int galic_set_targets(galic_ctx *ctx, int type, const double *dgs_mas
 }
 
 namespace {
-cudaError_t order_by_type_radius(galic_ctx *ctx);
+cudaError_t order_longest_first(galic_ctx *ctx);
 }
 
 extern "C" int galic_set_particles(galic_ctx *ctx, int n, const double *pos, const double *vel, const double *mass,
@@ -523,11 +523,7 @@ extern "C" int galic_set_particles(galic_ctx *ctx, int n, const double *pos, con
   CK(cudaMemcpyAsync(ctx->d_ptargets, targets, 4 * (size_t) n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_type, type, n * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(ctx->d_vdisp, 0, 4 * (size_t) n * sizeof(double), ctx->stream));
-  // by type, then by radius: neighbouring lanes then integrate orbits of one
-  // type (one velocity structure, no divergent projections) that start at
-  // similar radii and read nearby force-grid cells; results do not depend on
-  // the order.  Sorted on the GPU from the uploaded positions and types.
-  CK(order_by_type_radius(ctx));
+  CK(order_longest_first(ctx));
   CK(cudaMemsetAsync(ctx->d_orbits, 0, n * sizeof(int), ctx->stream));
   ctx->have_response = false;
   CK(cudaStreamSynchronize(ctx->stream));  // the upload is complete on return
@@ -546,56 +542,39 @@ __global__ void k_particle_meta(int n, int n1, int n12, double m1, double m2, do
   mass[i] = t == 1 ? m1 : (t == 2 ? m2 : m3);
 }
 
-// r^2 as it orders (non-negative doubles order like their bits)
-__global__ void k_radius_keys(int n, const double *pos, unsigned long long *key, int *idx)
+// the processing order: by length (kernels.cuh:orbit_length_class), then by
+// type (one velocity structure per warp), then by radius (lanes of a warp read
+// nearby force-grid cells)
+__global__ void k_order_keys(int n, const double *pos, const double *vel, const double *vesc, const int *type,
+                             unsigned long long *key, int *idx)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i >= n) return;
-  const double *p = pos + 3 * (size_t) i;
-  const double r2 = p[0] * p[0] + p[1] * p[1] + p[2] * p[2];
-  key[i] = (unsigned long long) __double_as_longlong(r2);
+  double r2;
+  const unsigned cls = orbit_length_class(pos + 3 * (size_t) i, vel + 3 * (size_t) i, vesc[i], &r2);
+  // non-negative doubles order like their bits (the sign bit is clear)
+  key[i] = ((unsigned long long) cls << 56) | ((unsigned long long) (type[i] & 3) << 54) |
+           ((unsigned long long) __double_as_longlong(r2) >> 9);
   idx[i] = i;
 }
 
-__global__ void k_type_keys(int n, const int *type, const int *idx, int *key)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= n) return;
-  key[i] = type[idx[i]];
-}
-
-// the orbit order (by type, then by radius, ties in index order) of the
-// context's particles into d_order: a stable radix sort by r^2, then a
-// stable one by type (1-3: two bits)
-cudaError_t order_by_type_radius(galic_ctx *ctx)
+// that order of the context's particles into d_order, ties in index order
+cudaError_t order_longest_first(galic_ctx *ctx)
 {
   const int n = ctx->n;
   cudaStream_t s = ctx->stream;
-  const unsigned g = (unsigned) ((n + 255) / 256);
-  unsigned long long *k0 = nullptr, *k1 = nullptr;
-  int *i0 = nullptr, *i1 = nullptr, *t0 = nullptr, *t1 = nullptr;
+  unsigned long long *k0 = nullptr;
+  int *i0 = nullptr;
   void *tmp = nullptr;
-  size_t tb = 0, tb2 = 0, tbx;
+  size_t tb = 0;
   cudaError_t e = cudaMallocAsync((void **) &k0, 2 * (size_t) n * sizeof(unsigned long long), s);
-  if(e == cudaSuccess) e = cudaMallocAsync((void **) &i0, 4 * (size_t) n * sizeof(int), s);
+  if(e == cudaSuccess) e = cudaMallocAsync((void **) &i0, (size_t) n * sizeof(int), s);
+  if(e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(nullptr, tb, k0, k0 + n, i0, ctx->d_order, n, 0, 64, s);
+  if(e == cudaSuccess) e = cudaMallocAsync(&tmp, std::max<size_t>(tb, 16), s);
   if(e == cudaSuccess) {
-    k1 = k0 + n;
-    i1 = i0 + n;
-    t0 = i1 + n;
-    t1 = t0 + n;
-    e = cub::DeviceRadixSort::SortPairs(nullptr, tb, k0, k1, i0, i1, n, 0, 64, s);
-  }
-  if(e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(nullptr, tb2, t0, t1, i1, ctx->d_order, n, 0, 2, s);
-  if(e == cudaSuccess) e = cudaMallocAsync(&tmp, std::max<size_t>(std::max(tb, tb2), 16), s);
-  if(e == cudaSuccess) {
-    k_radius_keys<<<g, 256, 0, s>>>(n, ctx->d_pos, k0, i0);
-    tbx = std::max(tb, tb2);
-    e = cub::DeviceRadixSort::SortPairs(tmp, tbx, k0, k1, i0, i1, n, 0, 64, s);
-  }
-  if(e == cudaSuccess) {
-    k_type_keys<<<g, 256, 0, s>>>(n, ctx->d_type, i1, t0);
-    tbx = std::max(tb, tb2);
-    e = cub::DeviceRadixSort::SortPairs(tmp, tbx, t0, t1, i1, ctx->d_order, n, 0, 2, s);
+    k_order_keys<<<(unsigned) ((n + 255) / 256), 256, 0, s>>>(n, ctx->d_pos, ctx->d_vel, ctx->d_vesc, ctx->d_type, k0,
+                                                              i0);
+    e = cub::DeviceRadixSort::SortPairs(tmp, tb, k0, k0 + n, i0, ctx->d_order, n, 0, 64, s);
   }
   if(e == cudaSuccess) e = cudaGetLastError();
   for(void *q : {(void *) k0, (void *) i0, tmp})
@@ -657,7 +636,7 @@ int set_particles_device(galic_ctx *ctx, const int nt[4], const double tmass[4],
                                                                 nt[2] ? tmass[2] / nt[2] : 0.0,
                                                                 nt[3] ? tmass[3] / nt[3] : 0.0, ctx->d_mass, ctx->d_type);
   CK(cudaGetLastError());
-  CK(order_by_type_radius(ctx));
+  CK(order_longest_first(ctx));
   ctx->have_response = false;
   CK(cudaStreamSynchronize(s));
   return fail(ctx, GALIC_OK);

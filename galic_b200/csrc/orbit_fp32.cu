@@ -450,9 +450,10 @@ struct SingleSrc {
   __device__ __forceinline__ const DevModel &model64(int) const { return M64; }
   __device__ __forceinline__ const Particles32 &particles(int) const { return P; }
   __device__ __forceinline__ int gridset(int, int type) const { return type; }
-  __device__ __forceinline__ bool take(int &mi, int &p) const
+  // the lane's first orbit (FirstOrbit), and orbit number k
+  __device__ __forceinline__ int first_orbit() const { return FirstOrbit().index; }
+  __device__ __forceinline__ bool take(int k, int &mi, int &p) const
   {
-    const int k = atomicAdd(next, 1);
     if(k >= n) return false;
     mi = 0;
     const int kk = first + k * stride;
@@ -491,9 +492,10 @@ struct EnsembleSrc {
   __device__ __forceinline__ const DevModel &model64(int mi) const { return mem[mi].dm; }
   __device__ __forceinline__ const Particles32 &particles(int mi) const { return mem[mi].part; }
   __device__ __forceinline__ int gridset(int mi, int type) const { return 4 * mi + type; }
-  __device__ __forceinline__ bool take(int &mi, int &p) const
+  // (consecutive orbits to the lanes of a warp here: they mostly share a model)
+  __device__ __forceinline__ int first_orbit() const { return (int) (blockIdx.x * blockDim.x + threadIdx.x); }
+  __device__ __forceinline__ bool take(int k, int &mi, int &p) const
   {
-    const int k = atomicAdd(next, 1);
     if(k >= total) return false;
     int lo = 0, hi = nmodels;
     while(hi - lo > 1) {
@@ -555,9 +557,9 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
   sink.cnt = 0;
   int mi = 0;
 
-  auto begin = [&]() -> bool {
+  auto begin = [&](int k) -> bool {
     int nmi, p;
-    if(!S.take(nmi, p)) {
+    if(!S.take(k, nmi, p)) {
       aux.p = -1;
       return false;
     }
@@ -592,7 +594,7 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
     return true;
   };
 
-  int state = begin() ? LANE_ACTIVE : LANE_DONE;
+  int state = begin(S.first_orbit()) ? LANE_ACTIVE : LANE_DONE;
   for(;;) {
     const bool all_done = !__any_sync(0xffffffffu, state != LANE_DONE);
     // records carry the orbit's grid set and scale only through the lane's
@@ -621,7 +623,7 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
       }
       state = LANE_START;
     } else if(state == LANE_START) {
-      state = begin() ? LANE_ACTIVE : LANE_DONE;
+      state = begin(FirstOrbit().lanes + atomicAdd(S.next, 1)) ? LANE_ACTIVE : LANE_DONE;
     }
   }
   S.flush_stats(aux.stat_mi, aux.steps, aux.err, aux.status);

@@ -273,9 +273,9 @@ __global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(con
   sink.cnt = 0;
   int p = -1;
 
-  // fetch the next orbit for this lane; returns false when none is left
-  auto fetch = [&]() -> bool {
-    int k = atomicAdd(A.next, 1);
+  // starts orbit number k of this launch on this lane; false when there is none
+  const FirstOrbit first;
+  auto fetch = [&](int k) -> bool {
     if(k >= A.n) {
       p = -1;
       return false;
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(con
     return true;
   };
 
-  int state = fetch() ? LANE_ACTIVE : LANE_DONE;
+  int state = fetch(first.index) ? LANE_ACTIVE : LANE_DONE;
   for(;;) {
     const bool all_done = !__any_sync(0xffffffffu, state != LANE_DONE);
     // records take the orbit's grid set and scale from the lane's queue
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(CALC_ALL_BLOCK_FP64, MINB) k_calc_all_fp64(con
       }
       state = LANE_START;
     } else if(state == LANE_START) {
-      state = fetch() ? LANE_ACTIVE : LANE_DONE;
+      state = fetch(first.lanes + atomicAdd(A.next, 1)) ? LANE_ACTIVE : LANE_DONE;
     }
   }
   __syncthreads();
