@@ -23,6 +23,7 @@ struct galic_ctx {
   // [2] the context's stream reached the call's start, [3], [4] a half's
   // orbits done
   cudaStream_t stream2 = nullptr;
+  cudaStream_t stream3 = nullptr;  // the orbits of every other window, while they are small
   cudaEvent_t ev2[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   int *d_idx_all = nullptr;               // every particle index of a galic_optimize_reps call
   size_t idx_cap = 0;

@@ -29,6 +29,23 @@
 #include "fixedpoint.cuh"
 #include "kernels.cuh"
 
+// The four nodes of a cell by parity: node (z, r) lives in slot
+// ((z & 1) << 1) | (r & 1), so that when an orbit moves to a neighbouring cell
+// the nodes the two cells share keep their slots.
+struct SlotNodes {
+  int z[2], r[2];  // the even and the odd node along each axis
+  __device__ __forceinline__ SlotNodes() : z{-1, -1}, r{-1, -1} {}
+  __device__ __forceinline__ SlotNodes(int iR, int iz) : z{(iz + 1) & ~1, iz | 1}, r{(iR + 1) & ~1, iR | 1} {}
+  __device__ __forceinline__ int index(int slot, int Nb) const { return z[slot >> 1] * Nb + r[slot & 1]; }
+  // out[slot]: the slot's node is not one of `next`
+  __device__ __forceinline__ void leaving(const SlotNodes &next, bool out[4]) const
+  {
+    const bool lz[2] = {z[0] != next.z[0], z[1] != next.z[1]}, lr[2] = {r[0] != next.r[0], r[1] != next.r[1]};
+#pragma unroll
+    for(int k = 0; k < 4; k++) out[k] = lz[k >> 1] || lr[k & 1];
+  }
+};
+
 // T: the type of the sums (float, double)
 template <int PER_, class T>
 struct WarpQueueT {

@@ -45,12 +45,21 @@ struct Model32 {
   long long step_cap;
 };
 
-__device__ __forceinline__ float frcp(float x) { return __frcp_rn(x); }
+__device__ __forceinline__ float frcp(float x) { return step_rcp32(x); }
 
 struct Cell32 {
   int iR, iz;
   float fR, fz;
 };
+
+// the two float4 of a 32-byte aligned sector in one load: one L1 request a
+// lookup instead of two
+__device__ __forceinline__ void load_pair(const float4 *p, float4 &a, float4 &b)
+{
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
 
 __device__ __forceinline__ Cell32 cell32(float br, float bz, int nbin, float bmax)
 {
@@ -81,7 +90,8 @@ __device__ __forceinline__ void accel32(const Model32 &M, int type, const float 
   Cell32 c = cell32(jd, id, N, M.fgmax);
   // corners in the quad: (iz,iR), (iz,iR+1), (iz+1,iR), (iz+1,iR+1)
   const float4 *Q = M.quad[type] + 4 * (c.iz * N + c.iR);
-  const float4 qR = __ldg(&Q[0]), qZ = __ldg(&Q[1]);
+  float4 qR, qZ;
+  load_pair(Q, qR, qZ);
   const float4 qV = M.vstream_zero[type] ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldg(&Q[2]);
   const float w00 = (1.f - c.fR) * (1.f - c.fz), w01 = c.fR * (1.f - c.fz);
   const float w10 = (1.f - c.fR) * c.fz, w11 = c.fR * c.fz;
@@ -164,36 +174,13 @@ __device__ __forceinline__ Cell32 density_cell32(const Model32 &M, const float *
   return cell32(br, bz, M.DG_Nbin, M.dgmax);
 }
 
-// Register-merged FP32 sums for the four grid nodes of the current DG cell.
-// A node (z, r) always lives in accumulator slot ((z & 1) << 1) | (r & 1):
-// the four nodes of any cell have the four parities, so when the orbit moves
-// to a neighbouring cell the nodes both cells share stay in their slots
-// untouched, and only the slots whose node changes are flushed and cleared.
-// A deposit's corner c = 2 dz + dr of the cell lands in slot c ^ (2 (iz & 1) + (iR & 1)).
+// Register-merged FP32 sums for the four grid nodes of the current DG cell, by
+// parity slot (flush.cuh:SlotNodes): when the orbit moves to a neighbouring cell
+// the nodes both cells share stay in their slots untouched, and only the
+// slots whose node changes are flushed and cleared.
 struct NodeAcc {
-  int cur = -1, cur_iR = 0, cur_iz = 0;
+  SlotNodes node;  // z[0] < 0: no cell yet
   float a[4][5];
-  // slot s of cell (iz, iR) holds node (iz + node_dz(s, iz), iR + node_dr(s, iR))
-  __device__ __forceinline__ static int node_dz(int s, int iz) { return ((s >> 1) ^ iz) & 1; }
-  __device__ __forceinline__ static int node_dr(int s, int iR) { return (s ^ iR) & 1; }
-  // slots whose node is not a node of cell (iz, iR)
-  __device__ __forceinline__ void leaving(int iR, int iz, bool out[4]) const
-  {
-    // along one axis a move by d leaves the node whose parity is that of the
-    // boundary left behind (d = +1: the lower node, d = -1: the upper one),
-    // both nodes when |d| > 1, none when d = 0
-    const int dz = iz - cur_iz, dr = iR - cur_iR;
-    const int bz = (dz > 0 ? cur_iz : cur_iz + 1) & 1, br = (dr > 0 ? cur_iR : cur_iR + 1) & 1;
-    const bool zall = dz > 1 || dz < -1, rall = dr > 1 || dr < -1;
-    bool lz[2], lr[2];
-#pragma unroll
-    for(int b = 0; b < 2; b++) {
-      lz[b] = zall || (dz != 0 && b == bz);
-      lr[b] = rall || (dr != 0 && b == br);
-    }
-#pragma unroll
-    for(int s = 0; s < 4; s++) out[s] = lz[s >> 1] || lr[s & 1];
-  }
   __device__ __forceinline__ void clear(const bool which[4])
   {
 #pragma unroll
@@ -228,20 +215,21 @@ struct Sink32 : NodeAcc {
   WarpQueue32<PER> *q;
   int lane, Nb;
   int cnt;  // records parked in this lane's queue column since the last drain
-  // the orbit's first word (grid set x NG_COMMITTED x Ngrid) and the scale
-  // factors mass/Tint x 2^(shift-24) of the mass and energy fields, kept in
-  // the lane's queue header (read only when parking)
+  // the orbit's grid set and the scale factors mass/Tint x 2^(shift-24) of
+  // the mass and energy fields, kept in the lane's queue header (read only by
+  // the drain)
   __device__ __forceinline__ void set_orbit(int gbase, float scale_m, float scale_e)
   {
     q->gbase[lane] = gbase;
     q->scale[0][lane] = scale_m;
     q->scale[1][lane] = scale_e;
+    const bool all[4] = {true, true, true, true};
+    clear(all);
   }
+  // parks the slots in out that hold a deposit (every field of a node is
+  // weight x ..., so one without mass has none)
   __device__ __forceinline__ void park_masked(const bool out[4])
   {
-    // a node with no mass has no deposit at all (every field is weight x ...);
-    // the records keep the raw sums and the node's index in the grid, the
-    // drain adds the orbit's grid set and scale factors
     bool rec[4];
     int at[4], k = cnt;
 #pragma unroll
@@ -253,7 +241,7 @@ struct Sink32 : NodeAcc {
 #pragma unroll
     for(int s = 0; s < 4; s++) {
       if(rec[s]) {
-        q->base[at[s]][lane] = (unsigned short) ((cur_iz + node_dz(s, cur_iz)) * Nb + cur_iR + node_dr(s, cur_iR));
+        q->base[at[s]][lane] = (unsigned short) node.index(s, Nb);
 #pragma unroll
         for(int f = 0; f < 5; f++) q->val[at[s]][f][lane] = a[s][f];
       }
@@ -262,43 +250,21 @@ struct Sink32 : NodeAcc {
   }
   __device__ __forceinline__ void park()
   {
-    if(cur < 0) return;
     const bool all[4] = {true, true, true, true};
     park_masked(all);
-    cur = -1;
   }
-  __device__ __forceinline__ void move_to(int iR, int iz)
-  {
-    if(cur >= 0) {
-      bool out[4];
-      leaving(iR, iz, out);
-      park_masked(out);
-      clear(out);
-    } else {
-      const bool all[4] = {true, true, true, true};
-      clear(all);
-    }
-    cur = iz * Nb + iR;
-    cur_iR = iR;
-    cur_iz = iz;
-  }
-  // straight-line form of `if(cell changed) move_to(iR, iz)`: every lane runs
-  // it (a warp nearly always has a lane whose cell changed), so the compiler
-  // can interleave it with the rest of the step; on an unchanged cell no
-  // slot leaves, on the orbit's first deposit every slot is cleared and
-  // nothing is parked
+  // straight-line code for every lane (a warp nearly always has a lane whose
+  // cell changed), so that it interleaves with the rest of the step; on an
+  // unchanged cell no slot leaves, and before an orbit's first deposit no slot
+  // holds anything
   __device__ __forceinline__ void add(int iR, int iz, float hdt, float fR, float fz, const Proj32 &p)
   {
-    const bool first = cur < 0;
+    const SlotNodes next(iR, iz);
     bool out[4];
-    leaving(iR, iz, out);
-#pragma unroll
-    for(int s = 0; s < 4; s++) out[s] = first || out[s];
-    if(!first) park_masked(out);
+    node.leaving(next, out);
+    park_masked(out);
     clear(out);
-    cur = iz * Nb + iR;
-    cur_iR = iR;
-    cur_iz = iz;
+    node = next;
     accumulate(iR, iz, hdt, fR, fz, p);
   }
 };
@@ -553,7 +519,6 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
   Sink32<PER> sink;
   sink.q = &queues[threadIdx.x >> 5];
   sink.lane = threadIdx.x & 31;
-  sink.cur = -1;
   sink.cnt = 0;
   int mi = 0;
 
@@ -582,7 +547,6 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
       sink.set_orbit(2 * gs * G, (float) ldexp(fac, S.shift[gs * NG_COMMITTED + GALIC_GRID_MASS_S] - 24),
                      (float) ldexp(fac, S.shift[gs * NG_COMMITTED + GALIC_GRID_R_S] - 24));
     }
-    sink.cur = -1;
     double xd[3], vd[3];
     for(int i = 0; i < 3; i++) {
       xd[i] = P.pos[3 * p + i];
@@ -649,39 +613,33 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_ensemble_fp32(const __grid_cons
 struct DenseSink32 : NodeAcc {
   double *grid;
   int G, Nb;
+  bool held = false;
   __device__ __forceinline__ void flush_nodes(const bool out[4])
   {
 #pragma unroll
     for(int s = 0; s < 4; s++) {
       if(!out[s]) continue;
-      const int node = (cur_iz + node_dz(s, cur_iz)) * Nb + cur_iR + node_dr(s, cur_iR);
+      const int at = node.index(s, Nb);
 #pragma unroll
       for(int f = 0; f < 5; f++)
-        if(a[s][f] != 0.f) atomicAdd(&grid[(size_t) f * G + node], (double) a[s][f]);
+        if(a[s][f] != 0.f) atomicAdd(&grid[(size_t) f * G + at], (double) a[s][f]);
     }
   }
   __device__ __forceinline__ void flush()
   {
-    if(cur < 0) return;
     const bool all[4] = {true, true, true, true};
-    flush_nodes(all);
-    cur = -1;
+    if(held) flush_nodes(all);
   }
   __device__ __forceinline__ void add(int iR, int iz, float hdt, float fR, float fz, const Proj32 &p)
   {
-    if(iz * Nb + iR != cur) {
-      if(cur >= 0) {
-        bool out[4];
-        leaving(iR, iz, out);
-        flush_nodes(out);
-        clear(out);
-      } else {
-        const bool all[4] = {true, true, true, true};
-        clear(all);
-      }
-      cur = iz * Nb + iR;
-      cur_iR = iR;
-      cur_iz = iz;
+    const SlotNodes next(iR, iz);
+    bool out[4];
+    node.leaving(next, out);
+    if(out[0] || out[1] || out[2] || out[3]) {
+      if(held) flush_nodes(out);
+      clear(out);
+      held = true;
+      node = next;
     }
     accumulate(iR, iz, hdt, fR, fz, p);
   }
@@ -693,8 +651,8 @@ struct DenseSink32 : NodeAcc {
 __global__ void __launch_bounds__(128) k_orbits_dense_fp32(const __grid_constant__ Model32 M,
                                                           const __grid_constant__ DevModel M64, OrbitBatch b)
 {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if(k >= b.count) return;
+  const int k = dense_orbit(b.count);
+  if(k < 0) return;
   const int G = M64.DG_Ngrid;
   DenseSink32 sink;
   sink.grid = b.grids + (size_t) k * NF_ORBIT * G;
@@ -823,7 +781,7 @@ void launch_orbits_dense_fp32(const DevModel &M64, const float4 *const quad[4], 
 {
   if(b.count <= 0) return;
   const Model32 M = make_model32(M64, quad, cellsize32);
-  k_orbits_dense_fp32<<<(b.count + 127) / 128, 128, 0, s>>>(M, M64, b);
+  k_orbits_dense_fp32<<<dense_grid(b.count, 128), 128, 0, s>>>(M, M64, b);
 }
 
 int ensemble_variant_count() { return kNumVariants; }

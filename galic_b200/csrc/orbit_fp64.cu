@@ -19,22 +19,6 @@
 
 namespace {
 
-// The four nodes of a cell by parity: node (z, r) lives in slot
-// ((z & 1) << 1) | (r & 1), so that when an orbit moves to a neighbouring cell
-// the nodes the two cells share keep their slots.
-struct SlotNodes {
-  int z[2], r[2];  // the even and the odd node along each axis
-  __device__ __forceinline__ SlotNodes() : z{-1, -1}, r{-1, -1} {}
-  __device__ __forceinline__ SlotNodes(int iR, int iz) : z{(iz + 1) & ~1, iz | 1}, r{(iR + 1) & ~1, iR | 1} {}
-  __device__ __forceinline__ int index(int slot, int Nb) const { return z[slot >> 1] * Nb + r[slot & 1]; }
-  // out[slot]: the slot's node is not one of `next`
-  __device__ __forceinline__ void leaving(const SlotNodes &next, bool out[4]) const
-  {
-    const bool lz[2] = {z[0] != next.z[0], z[1] != next.z[1]}, lr[2] = {r[0] != next.r[0], r[1] != next.r[1]};
-#pragma unroll
-    for(int k = 0; k < 4; k++) out[k] = lz[k >> 1] || lr[k & 1];
-  }
-};
 // the weights of a half step for cell c's nodes in slot order (products in
 // the order of orbit_response.c:277-320)
 __device__ __forceinline__ void slot_weights(const Cell &c, double hdt, double w[4])
@@ -124,8 +108,8 @@ struct DenseSink {
 
 __global__ void k_orbits_dense(const __grid_constant__ DevModel M, OrbitBatch b)
 {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if(k >= b.count) return;
+  const int k = dense_orbit(b.count);
+  if(k < 0) return;
   LogConsts L = step_log_consts(M);
   const size_t G = (size_t) M.DG_Ngrid;
   DenseSink sink;
@@ -379,8 +363,8 @@ __global__ void k_fx_finalize(const FxWord *fx, const int *shift, double *out, i
 void launch_orbits_dense(const DevModel &M, const OrbitBatch &b, cudaStream_t s)
 {
   int block = 64;
-  int grid = (b.count + block - 1) / block;
-  if(grid > 0) k_orbits_dense<<<grid, block, 0, s>>>(M, b);
+  const int grid = dense_grid(b.count, block);
+  if(b.count > 0) k_orbits_dense<<<grid, block, 0, s>>>(M, b);
 }
 
 void launch_scale_dense(const DevModel &M, const OrbitBatch &b, cudaStream_t s)

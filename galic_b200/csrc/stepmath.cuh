@@ -130,6 +130,18 @@ __device__ __forceinline__ void step_direction(double y, double x, double *s, do
   *c = tiny ? 1.0 : (((n.i + 1) & 2) ? -cv : cv);
 }
 
+// __frcp_rn(x) with flushed subnormals (-ftz=true) without its branch: one
+// Newton step from the hardware's approximation is the correctly rounded
+// reciprocal of every normal x (tests/test_step_math.py compares all 2^32
+// arguments); 0 and infinity, whose residual is NaN, keep the approximation.
+__device__ __forceinline__ float step_rcp32(float x)
+{
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  const float r = __fmaf_rn(-x, y, 1.f);
+  return r == r ? __fmaf_rn(r, y, y) : y;
+}
+
 // true when every |c[i]| is in [2^-100, 2^100)
 __device__ __forceinline__ bool step_safe(const double *c)
 {

@@ -41,6 +41,24 @@ __global__ void k_cmp(int n, const double *a, const double *b, int what, unsigne
   }
   if(!ok) atomicAdd(bad, 1u);
 }
+__global__ void k_rcp32(unsigned *bad)
+{
+  const unsigned long long stride = (unsigned long long) gridDim.x * blockDim.x;
+  for(unsigned long long u = blockIdx.x * (unsigned long long) blockDim.x + threadIdx.x; u < (1ULL << 32); u += stride) {
+    const float x = __uint_as_float((unsigned) u), a = step_rcp32(x), b = __frcp_rn(x);
+    if(__float_as_uint(a) != __float_as_uint(b) && (a == a || b == b)) atomicAdd(bad, 1u);
+  }
+}
+extern "C" int compare_rcp32(void)
+{
+  unsigned *bad, h = 0;
+  if(cudaMalloc(&bad, 4)) return -1;
+  cudaMemset(bad, 0, 4);
+  k_rcp32<<<148 * 8, 256>>>(bad);
+  if(cudaMemcpy(&h, bad, 4, cudaMemcpyDeviceToHost)) return -1;
+  cudaFree(bad);
+  return (int) h;
+}
 extern "C" int compare(int n, const double *a, const double *b, int what)
 {
   double *da, *db;
@@ -62,7 +80,7 @@ def lib(tmp_path_factory):
     d = tmp_path_factory.mktemp("step")
     (d / "t.cu").write_text(SRC)
     subprocess.run(["/usr/local/cuda/bin/nvcc", "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a",
-                    "--fmad=false", "-shared", "-Xcompiler", "-fPIC", "-I", os.path.join(ROOT, "galic_b200", "csrc"),
+                    "--fmad=false", "-ftz=true", "-shared", "-Xcompiler", "-fPIC", "-I", os.path.join(ROOT, "galic_b200", "csrc"),
                     str(d / "t.cu"), "-o", str(d / "libt.so")], check=True)
     return C.CDLL(str(d / "libt.so"))
 
@@ -108,6 +126,11 @@ def test_step_functions_equal_the_general_ones(lib, what):
     a, b = np.ascontiguousarray(a, dtype=np.float64), np.ascontiguousarray(b, dtype=np.float64)
     P = C.POINTER(C.c_double)
     assert lib.compare(len(a), a.ctypes.data_as(P), b.ctypes.data_as(P), what) == 0
+
+
+@pytest.mark.gpu
+def test_step_rcp32_equals_the_rounded_reciprocal_everywhere(lib):
+    assert lib.compare_rcp32() == 0
 
 
 @pytest.mark.gpu
