@@ -29,7 +29,7 @@ typedef struct {
   uint32_t key[2];
   uint32_t ctr[4];   /* ctr[0..1]: block counter, ctr[2..3]: stream id */
   uint32_t buf[4];
-  int have;          /* number of unused 32-bit words in buf (0, 2 or 4) */
+  int have;          /* number of unused 32-bit words in buf (0 or 2) */
 } grng_t;
 
 GM_HD void grng_mulhilo(uint32_t a, uint32_t b, uint32_t *hi, uint32_t *lo)
@@ -70,17 +70,22 @@ GM_HD void grng_init(grng_t *g, uint64_t seed, uint32_t stream_a, uint32_t strea
   g->have = 0;
 }
 
-/* uniform double in [0,1) with 53 random bits */
+/* uniform double in [0,1) with 53 random bits: the words 0, 1 of a block, then
+ * 2, 3 (constant indices, so that a GPU thread keeps the state in registers) */
 GM_HD double grng_uniform(grng_t *g)
 {
+  uint32_t a, b;
   if(g->have == 0) {
     grng_philox(g->ctr, g->key, g->buf);
     if(++g->ctr[0] == 0) ++g->ctr[1];
-    g->have = 4;
+    a = g->buf[0];
+    b = g->buf[1];
+    g->have = 2;
+  } else {
+    a = g->buf[2];
+    b = g->buf[3];
+    g->have = 0;
   }
-  uint32_t a = g->buf[4 - g->have];
-  uint32_t b = g->buf[5 - g->have];
-  g->have -= 2;
   uint64_t bits = (((uint64_t) a << 32) | (uint64_t) b) >> 11;
   return (double) bits * 0x1.0p-53;
 }

@@ -39,9 +39,12 @@ __device__ __forceinline__ bool halo_draw(const Shape &S, double q, double uphi,
     r = 0;
   double phi = uphi * kPi * 2;
   double theta = gm_acos(uth * 2 - 1);
-  pos[0] = r * gm_sin(theta) * gm_cos(phi);
-  pos[1] = r * gm_sin(theta) * gm_sin(phi);
-  pos[2] = r * gm_cos(theta) / S.HaloStretch;
+  double st, ct, sp, cp;
+  gm_sincos(theta, &st, &ct);  // gm_sin, gm_cos without their branches
+  gm_sincos(phi, &sp, &cp);
+  pos[0] = r * st * cp;
+  pos[1] = r * st * sp;
+  pos[2] = r * ct / S.HaloStretch;
   r = sqrt(pos[0] * pos[0] + pos[1] * pos[1] + pos[2] * pos[2]);
   return !(r > S.Rmax);
 }
@@ -61,8 +64,10 @@ __device__ __forceinline__ bool disk_draw(const Shape &S, double q1, double q2, 
   } while(gm_fabs(R - Rold) / R > 1e-7 && ++it < NEWTON_CAP);
   R *= S.Disk_H;
   double phi = uphi * kPi * 2;
-  pos[0] = R * gm_cos(phi);
-  pos[1] = R * gm_sin(phi);
+  double sp, cp;
+  gm_sincos(phi, &sp, &cp);
+  pos[0] = R * cp;
+  pos[1] = R * sp;
   double R2 = pos[0] * pos[0] + pos[1] * pos[1] + pos[2] * pos[2];
   return !(R2 > S.Rmax * S.Rmax);
 }
@@ -78,9 +83,12 @@ __device__ __forceinline__ void bulge_place(const Shape &S, double r, double uph
 {
   double phi = uphi * kPi * 2;
   double theta = gm_acos(uth * 2 - 1);
-  pos[0] = r * gm_sin(theta) * gm_cos(phi);
-  pos[1] = r * gm_sin(theta) * gm_sin(phi);
-  pos[2] = r * gm_cos(theta) / S.BulgeStretch;
+  double st, ct, sp, cp;
+  gm_sincos(theta, &st, &ct);
+  gm_sincos(phi, &sp, &cp);
+  pos[0] = r * st * cp;
+  pos[1] = r * st * sp;
+  pos[2] = r * ct / S.BulgeStretch;
 }
 
 // ---------------------------------------------------------------- dispersions

@@ -275,3 +275,22 @@ def test_gpu_sampled_targets_drive_calc_all():
     L = m.params.DG_MaxLevel
     off = ((1 << (2 * L)) - 1) // 3
     assert abs(np.sum(dg[off:]) - m.params.MType[1]) < 1e-9 * m.params.MType[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntarget", [2, 31, 33, 64 * 32 + 1])
+@pytest.mark.parametrize("level", [4, 7])
+def test_gpu_targets_at_warp_edges(ntarget, level):
+    # counts that end inside a warp's row of samples, where its words are added together
+    m = composite(level=level)
+    sp = shape(m, Rmax=0.3 * m.meta["rmax"], HaloStretch=1.2)
+    tables = disp_tables(m, 5)
+    for kind, first in (("density", 0), ("energy", 1)):
+        stream = (17, 1, 0, 5)
+        got, gpos, _ = _gpu_targets(m, sp, ntarget, stream, kind, tables)
+        ref, rpos = _restatement_targets(m, sp, ntarget, stream, kind, use_libm=False, tables=tables)
+        assert gpos == rpos
+        for t in (1, 2, 3):
+            rt = ref[t] if first else [ref[t]]
+            for k in range(len(rt)):
+                assert peak_rel(got[t][first + k], rt[k]) < 1e-12, (kind, t, k)
