@@ -145,13 +145,13 @@ int ensure_rep_scratch(galic_ctx *ctx, int count)
   int st = ensure_orbit_scratch(ctx, 2 * count);
   if(st) return st;
   if(count <= ctx->scratch_rep) return GALIC_OK;
-  dfree(ctx, ctx->d_idx); dfree(ctx, ctx->d_accepted); dfree(ctx, ctx->d_vel_try); dfree(ctx, ctx->d_F); dfree(ctx, ctx->d_inst_v);
+  dfree(ctx, ctx->d_idx); dfree(ctx, ctx->d_vel_try); dfree(ctx, ctx->d_F); dfree(ctx, ctx->d_inst_v);
   dfree(ctx, ctx->d_inst_cell); dfree(ctx, ctx->d_acc_list); dfree(ctx, ctx->d_acc_n); dfree(ctx, ctx->d_fac);
+  dfree(ctx, ctx->d_try_disp);
   CK(dalloc(ctx, &ctx->d_idx, count));
-  CK(dalloc(ctx, &ctx->d_acc_list, count));
-  CK(dalloc(ctx, &ctx->d_acc_n, count));  // one per repetition: at most count repetitions per window
-  if(!ctx->d_inst0) CK(dalloc(ctx, &ctx->d_inst0, 16));
-  CK(dalloc(ctx, &ctx->d_accepted, count));
+  CK(dalloc(ctx, &ctx->d_acc_list, 3 * (size_t) count));
+  CK(dalloc(ctx, &ctx->d_acc_n, 3 * (size_t) count));  // one per repetition: at most count repetitions per window
+  CK(dalloc(ctx, &ctx->d_try_disp, 4 * (size_t) count));
   CK(dalloc(ctx, &ctx->d_vel_try, 3 * (size_t) count));
   CK(dalloc(ctx, &ctx->d_F, 2 * 9 * (size_t) count));  // 9 merit terms per evaluation
   CK(dalloc(ctx, &ctx->d_fac, 2 * (size_t) count));
@@ -176,7 +176,10 @@ FitArgs make_fit_args(galic_ctx *ctx)
   f.stacks = ctx->d_stacks;
   f.targets = ctx->d_targets;
   f.dgs_distance = ctx->d_dist;
+  f.values = ctx->d_stacks + (size_t) 4 * NG_COMMITTED * ctx->Ns;
   f.fit = ctx->d_fit;
+  f.raw = ctx->d_fit + 4 * 7;
+  f.arrived = (unsigned *) (ctx->d_fit + 4 * 7 + 4 * 5);
   f.firstrun = ctx->d_firstrun;
   for(int t = 0; t < 4; t++) {
     // main.c:296 / 313: MinParticles * MType / NType, left to right
@@ -304,7 +307,6 @@ int galic_internal::ctx_create(const galic_params_t *prm, int priority, galic_ct
   ctx->priority = priority;
   CK(cudaStreamCreateWithPriority(&ctx->stream, cudaStreamNonBlocking, priority));
   for(int k = 0; k < 3; k++) CK(cudaEventCreate(&ctx->ev[k]));
-  CK(prepare_fit_kernels());
   ctx->L = prm->DG_MaxLevel;
   ctx->G = 1 << (2 * ctx->L);
   ctx->Ns = stack_size(ctx->L);
@@ -323,11 +325,11 @@ int galic_internal::ctx_create(const galic_params_t *prm, int priority, galic_ct
   CK(cudaMemsetAsync(ctx->d_targets, 0, (size_t) 4 * NT_TARGET * ctx->Ns * sizeof(double), ctx->stream));
   CK(dalloc(ctx, &ctx->d_committed, (size_t) 4 * NG_COMMITTED * ctx->G));
   CK(cudaMemsetAsync(ctx->d_committed, 0, (size_t) 4 * NG_COMMITTED * ctx->G * sizeof(double), ctx->stream));
-  CK(dalloc(ctx, &ctx->d_stacks, (size_t) 4 * NG_COMMITTED * ctx->Ns));
+  CK(dalloc(ctx, &ctx->d_stacks, (size_t) 4 * (NG_COMMITTED + FIT_TERMS) * ctx->Ns));
   CK(dalloc(ctx, &ctx->d_fx, (size_t) 4 * NG_COMMITTED * ctx->G));
   CK(dalloc(ctx, &ctx->d_shift, 4 * NG_COMMITTED));
-  CK(dalloc(ctx, &ctx->d_fit, 4 * 7 + 4 * 5));
-  CK(cudaMemsetAsync(ctx->d_fit, 0, (4 * 7 + 4 * 5) * sizeof(double), ctx->stream));
+  CK(dalloc(ctx, &ctx->d_fit, 4 * 7 + 4 * 5 + 2));
+  CK(cudaMemsetAsync(ctx->d_fit, 0, (4 * 7 + 4 * 5 + 2) * sizeof(double), ctx->stream));
   CK(dalloc(ctx, &ctx->d_firstrun, 4));
   CK(cudaMemsetAsync(ctx->d_firstrun, 0, 4 * sizeof(int), ctx->stream));
   CK(dalloc(ctx, &ctx->d_counters, 9));
@@ -398,8 +400,8 @@ extern "C" void galic_ctx_destroy(galic_ctx *ctx)
   dfree(ctx, ctx->d_b_pos); dfree(ctx, ctx->d_b_vel); dfree(ctx, ctx->d_b_mass); dfree(ctx, ctx->d_b_time); dfree(ctx, ctx->d_grids);
   dfree(ctx, ctx->d_b_tall); dfree(ctx, ctx->d_b_err); dfree(ctx, ctx->d_b_type); dfree(ctx, ctx->d_b_norbit); dfree(ctx, ctx->d_b_status);
   dfree(ctx, ctx->d_b_steps);
-  dfree(ctx, ctx->d_idx); dfree(ctx, ctx->d_accepted); dfree(ctx, ctx->d_vel_try); dfree(ctx, ctx->d_F); dfree(ctx, ctx->d_inst_v);
-  dfree(ctx, ctx->d_inst_cell); dfree(ctx, ctx->d_acc_list); dfree(ctx, ctx->d_acc_n); dfree(ctx, ctx->d_inst0);
+  dfree(ctx, ctx->d_idx); dfree(ctx, ctx->d_vel_try); dfree(ctx, ctx->d_F); dfree(ctx, ctx->d_inst_v);
+  dfree(ctx, ctx->d_inst_cell); dfree(ctx, ctx->d_acc_list); dfree(ctx, ctx->d_acc_n); dfree(ctx, ctx->d_try_disp);
   dfree(ctx, ctx->d_fac); dfree(ctx, ctx->d_idx_all); dfree(ctx, ctx->d_fit_hist); dfree(ctx, ctx->d_rep_stats);
   for(int t = 0; t < 4; t++) dfree(ctx, ctx->d_tab32[t]);
   dfree(ctx, ctx->d_cellsize32);
@@ -821,7 +823,7 @@ int enqueue_orbits(galic_ctx *ctx, int form, int first, int stride, int *launche
 // fixed point -> committed grids, then calc_global_fit (main.c:251-362)
 int enqueue_finish(galic_ctx *ctx, int form, int *launches)
 {
-  launch_fx_finalize(ctx->d_fx, ctx->d_shift, ctx->d_committed, 4 * NG_COMMITTED, ctx->G, form, ctx->stream);
+  launch_fx_finalize(ctx->d_fx, ctx->d_shift, ctx->d_committed, 4, 0, NG_COMMITTED, ctx->G, form, ctx->stream);
   *launches += 1;
   *launches += launch_global_fit(make_fit_args(ctx), ctx->stream);
   CK(cudaGetLastError());
@@ -944,10 +946,9 @@ RepArgs make_rep_args(galic_ctx *ctx, int count, uint64_t seed, uint32_t rep_ser
   R.fac = ctx->d_fac;
   R.vel_try = ctx->d_vel_try;
   R.F = ctx->d_F;
-  R.accepted = ctx->d_accepted;
   R.acc_list = ctx->d_acc_list;
   R.acc_n = ctx->d_acc_n;
-  R.inst0 = ctx->d_inst0;
+  R.try_disp = ctx->d_try_disp;
   R.inst_v = ctx->d_inst_v;
   R.inst_cell = ctx->d_inst_cell;
   R.tries = ctx->d_counters;
@@ -1142,11 +1143,7 @@ extern "C" int galic_optimize_reps(galic_ctx *ctx, const int *idx, int count, in
       ctx->fit_hist_cap = reps;
     }
   }
-  auto record_fit = [&](int r) -> cudaError_t {
-    if(!fits) return cudaSuccess;
-    return cudaMemcpyAsync(ctx->d_fit_hist + (size_t) r * 28, ctx->d_fit, 28 * sizeof(double),
-                           cudaMemcpyDeviceToDevice, s);
-  };
+  auto hist = [&](int r) { return fits ? ctx->d_fit_hist + (size_t) r * 28 : nullptr; };
   auto copy_fits = [&]() -> int {
     if(!fits || reps == 0) return GALIC_OK;
     CK(cudaMemcpyAsync(fits, ctx->d_fit_hist, (size_t) reps * 28 * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1155,8 +1152,7 @@ extern "C" int galic_optimize_reps(galic_ctx *ctx, const int *idx, int count, in
   };
   if(count == 0) {
     for(int r = 0; r < reps; r++) {
-      launches += launch_global_fit(f, s);
-      CK(record_fit(r));
+      launches += launch_global_fit(f, s, hist(r));
     }
     int st = copy_fits();
     if(st) return st;
@@ -1230,6 +1226,7 @@ extern "C" int galic_optimize_reps(galic_ctx *ctx, const int *idx, int count, in
   const OrbitBatch ball = make_rep_batch(ctx, nbuf * maxM);
   unsigned long long *d_total = (unsigned long long *) ctx->d_rep_stats;
   int *d_worst = (int *) (ctx->d_rep_stats + 1);
+  launches += launch_rep_values(f, s);
   for(size_t w = 0; w < wins.size(); w++) {
     cudaStream_t so = pair && (w & 1) ? ctx->stream3 : ctx->stream2;
     const int half = (int) (w % nbuf), W = wins[w].r1 - wins[w].r0, M = W * count;
@@ -1254,8 +1251,7 @@ extern "C" int galic_optimize_reps(galic_ctx *ctx, const int *idx, int count, in
     // each repetition's evaluation against the state its predecessors
     // committed, acceptance and commit, in order
     for(int j = 0; j < W; j++) {
-      launches += launch_rep_commit(ctx->dm, rep_slice(R, j * count, count, ctx->G), f, s);
-      CK(record_fit(wins[w].r0 + j));
+      launches += launch_rep_commit(ctx->dm, rep_slice(R, j * count, count, ctx->G), f, s, hist(wins[w].r0 + j));
     }
     k_window_stats<<<(b.count + 255) / 256 < 148 ? (b.count + 255) / 256 : 148, 256, 0, s>>>(b.steps, b.status,
                                                                                              b.count, d_total, d_worst);

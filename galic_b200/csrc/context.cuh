@@ -38,10 +38,10 @@ struct galic_ctx {
   double *d_cellsize = nullptr, *d_dist = nullptr;
   double *d_targets = nullptr;    // [4][6][Ns]
   double *d_committed = nullptr;  // [4][10][G]
-  double *d_stacks = nullptr;     // [4][10][Ns]
+  double *d_stacks = nullptr;     // [4][10][Ns], then the node values [4][9][Ns]
   FxWord *d_fx = nullptr;         // [4][10][G]
   int *d_shift = nullptr;         // [4][10]
-  double *d_fit = nullptr;        // [4][7] + raw [4][5]
+  double *d_fit = nullptr;        // [4][7] + raw [4][5] + 4 counters
   int *d_firstrun = nullptr;      // [4]
   unsigned long long *d_counters = nullptr;  // tries[4], changes[4], steps
   int *d_status = nullptr;
@@ -63,8 +63,8 @@ struct galic_ctx {
   int *d_b_type = nullptr, *d_b_norbit = nullptr, *d_b_status = nullptr;
   long long *d_b_steps = nullptr;
   int scratch_rep = 0;
-  int *d_idx = nullptr, *d_accepted = nullptr, *d_acc_list = nullptr, *d_acc_n = nullptr;
-  double *d_vel_try = nullptr, *d_F = nullptr, *d_inst_v = nullptr, *d_inst0 = nullptr, *d_fac = nullptr;
+  int *d_idx = nullptr, *d_acc_list = nullptr, *d_acc_n = nullptr;
+  double *d_vel_try = nullptr, *d_F = nullptr, *d_inst_v = nullptr, *d_try_disp = nullptr, *d_fac = nullptr;
   Cell *d_inst_cell = nullptr;
   // diagnostics
   long long last_steps = 0;

@@ -36,7 +36,8 @@ struct galic_ensemble {
   int G = 0;
   std::vector<galic_ctx *> members;
   std::vector<unsigned> generation;
-  cudaStream_t stream = nullptr;
+  cudaStream_t stream = nullptr, side = nullptr;
+  cudaEvent_t fork[2] = {nullptr, nullptr};
   EnsembleLaunch L{};
   void *d_members = nullptr;
   int *d_next = nullptr;
@@ -120,15 +121,26 @@ int enqueue_iteration(galic_ensemble *e, int variant, int grid)
   ECK(cudaMemsetAsync(e->d_maxerr, 0, e->nmodels * sizeof(double), s));
   ECK(cudaMemsetAsync(e->d_status, 0, e->nmodels * sizeof(int), s));
   ECK(cudaEventRecordWithFlags(e->ev[1], s, cudaEventRecordExternal));
-  ECK(launch_ensemble_fp32(e->L, variant, grid, s));
-  ECK(cudaEventRecordWithFlags(e->ev[2], s, cudaEventRecordExternal));
+  // the instantaneous fields and their misfits need no orbit: a branch beside it
+  ECK(cudaEventRecord(e->fork[0], s));
+  ECK(cudaStreamWaitEvent(e->side, e->fork[0], 0));
   for(int m = 0; m < e->nmodels; m++) {
     galic_ctx *c = e->members[m];
     FxWord *fx = e->d_fx + (size_t) m * 4 * NG_COMMITTED * e->G;
     const int *shift = e->d_shift + m * 4 * NG_COMMITTED;
-    launch_instantaneous(c->dm, c->n, c->d_pos, c->d_vel, c->d_mass, c->d_type, c->d_vdisp, fx, shift, e->G, s);
-    launch_fx_finalize(fx, shift, c->d_committed, 4 * NG_COMMITTED, e->G, GALIC_FORM_FP32, s);
-    launch_global_fit(make_fit_args(c), s);
+    launch_instantaneous(c->dm, c->n, c->d_pos, c->d_vel, c->d_mass, c->d_type, c->d_vdisp, fx, shift, e->G, e->side);
+    launch_fx_finalize(fx, shift, c->d_committed, 4, NF_ORBIT, NG_COMMITTED - NF_ORBIT, e->G, GALIC_FORM_FP32, e->side);
+    launch_global_fit(make_fit_args(c), e->side, nullptr, 5, FIT_TERMS - 5);
+  }
+  ECK(cudaEventRecord(e->fork[1], e->side));
+  ECK(launch_ensemble_fp32(e->L, variant, grid, s));
+  ECK(cudaEventRecordWithFlags(e->ev[2], s, cudaEventRecordExternal));
+  ECK(cudaStreamWaitEvent(s, e->fork[1], 0));
+  for(int m = 0; m < e->nmodels; m++) {
+    galic_ctx *c = e->members[m];
+    launch_fx_finalize(e->d_fx + (size_t) m * 4 * NG_COMMITTED * e->G, e->d_shift + m * 4 * NG_COMMITTED, c->d_committed, 4,
+                       0, NF_ORBIT, e->G, GALIC_FORM_FP32, s);
+    launch_global_fit(make_fit_args(c), s, nullptr, 0, 5);
   }
   ECK(cudaGetLastError());
   ECK(cudaEventRecordWithFlags(e->ev[3], s, cudaEventRecordExternal));
@@ -196,6 +208,8 @@ int ensemble_setup(galic_ensemble *e, galic_ctx *const *members, int count, int 
   e->G = G;
   e->members.assign(members, members + count);
   ECK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
+  ECK(cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking));
+  for(int k = 0; k < 2; k++) ECK(cudaEventCreateWithFlags(&e->fork[k], cudaEventDisableTiming));
   for(int k = 0; k < 4; k++) ECK(cudaEventCreate(&e->ev[k]));
   const size_t mb = ensemble_member_bytes();
   std::vector<char> host_members(mb * count);
@@ -238,7 +252,6 @@ int ensemble_setup(galic_ensemble *e, galic_ctx *const *members, int count, int 
   L.steps = e->d_steps;
   L.maxerr = e->d_maxerr;
   L.status = e->d_status;
-  ECK(prepare_fit_kernels());
   return GALIC_OK;
 }
 
@@ -261,6 +274,9 @@ extern "C" void galic_ensemble_destroy(galic_ensemble *e)
   cudaFreeHost(e->h_status);
   for(int k = 0; k < 4; k++)
     if(e->ev[k]) cudaEventDestroy(e->ev[k]);
+  for(int k = 0; k < 2; k++)
+    if(e->fork[k]) cudaEventDestroy(e->fork[k]);
+  if(e->side) cudaStreamDestroy(e->side);
   if(e->stream) cudaStreamDestroy(e->stream);
   delete e;
 }

@@ -1,21 +1,21 @@
 // Merit function and optimisation repetition (built with --fmad=false).
 //
-//  k_fit_smooth / k_fit_diff / k_fit_final   calc_global_fit (main.c:251-362)
+//  k_fit          calc_global_fit (main.c:251-362), one CTA per type and term
 //  k_propose      the proposal part of optimize (main.c:365-441)
-//  k_eval_terms   the nine stack terms of eval_fit_mod (main.c:1021-1217), one
-//                 CTA per term of each evaluation; k_accept combines them
-//  k_accept       the accept branch of optimize (main.c:468-507)
-//  k_delta_cols   the _delta accumulation (main.c:477-486) and commit_updates
-//                 (main.c:818-827): per bin, the accepted particles'
-//                 new - old values are summed in particle order, as the
-//                 reference's sequential loop does, then added to the
+//  k_eval_terms   the nine stack terms of eval_fit_mod (main.c:1021-1217)
+//  k_accept       their combination, the accept branch of optimize
+//                 (main.c:468-507) and the accepted positions in order
+//  k_commit       the _delta accumulation (main.c:477-486), add_to_energy_grid
+//                 of the accepted particles (main.c:488-498) and
+//                 commit_updates (main.c:818-835): per bin, the accepted
+//                 particles' new - old values are summed in particle order,
+//                 as the reference's sequential loop does, then added to the
 //                 committed grid.
-//  k_compact      the accepted positions of a repetition, in order
-//  k_inst_delta   add_to_energy_grid of the accepted particles
-//                 (main.c:488-498) and its commit (main.c:830-835).
+//
+// A repetition's commit is a chain of these kernels on one stream, each a few
+// microseconds long, and the next repetition waits for it: latency is what it
+// costs.
 #include <cuda_runtime.h>
-
-#include <mutex>
 
 #include "galic_gpu.h"
 #include "grng.h"
@@ -25,64 +25,87 @@
 
 namespace {
 
-__global__ void __launch_bounds__(1024) k_fit_smooth(FitArgs f)
-{
-  extern __shared__ double sm[];
-  const int type = blockIdx.x / NG_COMMITTED, g = blockIdx.x % NG_COMMITTED;
-  if(type < 1 || !f.present[type]) return;
-  const int off = ((1 << (2 * f.L)) - 1) / 3;
-  const double *src = f.committed + ((size_t) type * NG_COMMITTED + g) * f.Ngrid;
-  for(int i = threadIdx.x; i < f.Ngrid; i += blockDim.x) sm[off + i] = src[i];
-  __syncthreads();
-  stack_smooth_cta(sm, f.L);
-  double *dst = f.stacks + ((size_t) type * NG_COMMITTED + g) * f.Nstack;
-  for(int i = threadIdx.x; i < f.Nstack; i += blockDim.x) dst[i] = sm[i];
-}
+// The nine terms of the merit function.  0: density (main.c:1033-1047); 1-4:
+// the time-averaged dispersions r, t, q, p (main.c:1052-1120); 5-8: the
+// instantaneous ones r, t, p, q (main.c:1125-1176).
+enum { NTERM = FIT_TERMS };
+__device__ __constant__ const int kTermGrid[NTERM] = {GALIC_GRID_MASS_S, GALIC_GRID_R_S, GALIC_GRID_T_S,
+                                                      GALIC_GRID_Q_S,    GALIC_GRID_P_S, GALIC_GRID_R_I,
+                                                      GALIC_GRID_T_I,    GALIC_GRID_P_I, GALIC_GRID_Q_I};
+__device__ __constant__ const int kTermTarget[NTERM] = {T_DGM, T_R, T_T, T_Q, T_P, T_R, T_T, T_P, T_Q};
 
-// raw[type][w]: w = 0 S, 1 Sdisp_r, 2 Sdisp_t, 3 Sdisp_p, 4 Sdisp_q
-__global__ void __launch_bounds__(1024) k_fit_diff(FitArgs f, double *raw)
-{
-  extern __shared__ double sm[];
-  const int type = blockIdx.x / 5, w = blockIdx.x % 5;
-  if(type < 1 || !f.present[type]) return;
-  const double *stk = f.stacks + (size_t) type * NG_COMMITTED * f.Nstack;
-  const double *tg = f.targets + (size_t) type * NT_TARGET * f.Nstack;
-  const double *d1, *d2, *r1, *r2, *dist;
-  double thr;
-  int flag;
-  if(w == 0) {
-    d1 = stk + (size_t) GALIC_GRID_MASS_S * f.Nstack;
-    d2 = tg + (size_t) T_DGM * f.Nstack;
-    r1 = d2;
-    r2 = nullptr;
+// KIND 0: term 0, 1: terms 1-4, 2: terms 5-8
+template <int KIND>
+struct TermLeaf {
+  const double *d2, *r2, *dist;
+  double R200_20, lowdisp;
+  __device__ __forceinline__ TermLeaf(const FitArgs &f, int type, int term)
+  {
+    const double *tg = f.targets + (size_t) type * NT_TARGET * f.Nstack;
+    d2 = tg + (size_t) kTermTarget[term] * f.Nstack;
+    r2 = KIND == 2 ? tg + (size_t) T_EGM * f.Nstack : d2;
     dist = f.dgs_distance;
-    thr = f.thr_d[type];
-    flag = 0;
-  } else {
-    const int gi[5] = {0, GALIC_GRID_R_I, GALIC_GRID_T_I, GALIC_GRID_P_I, GALIC_GRID_Q_I};
-    const int ti[5] = {0, T_R, T_T, T_P, T_Q};
-    d1 = stk + (size_t) gi[w] * f.Nstack;
-    d2 = tg + (size_t) ti[w] * f.Nstack;
-    r1 = stk + (size_t) GALIC_GRID_MASS_I * f.Nstack;
-    r2 = tg + (size_t) T_EGM * f.Nstack;
-    dist = nullptr;
-    thr = f.thr_e[type];
-    flag = 1;
+    R200_20 = f.R200_20;
+    lowdisp = f.LowerDispLimit;
   }
-  for(int i = threadIdx.x; i < f.Nstack; i += blockDim.x) sm[i] = d1[i];
-  __syncthreads();
-  double v = stack_diff_cta(sm, d2, r1, r2, dist, thr, flag, 0, f.L, f.R200_20, f.LowerDispLimit);
-  if(threadIdx.x == 0) raw[type * 5 + w] = v;
+  __device__ __forceinline__ double operator()(int node, double d1, double r1) const
+  {
+    return stack_leaf(d1, d2[node], r1, KIND ? r2[node] : 0.0, KIND == 2 ? 0.0 : dist[node], KIND == 0 ? 0 : 3 - KIND,
+                      KIND == 1, R200_20, lowdisp);
+  }
+};
+
+// from_stacks: the finest level is the stacks' (the values of their nodes are
+// wanted for k_eval_terms, nothing else changes)
+template <int KIND>
+__device__ __forceinline__ double fit_term(const FitArgs &f, int type, int term, bool from_stacks,
+                                           Pyramid<1, KIND == 2> &sm)
+{
+  const int L = f.L, N = 1 << L, Ns = f.Nstack, off = stack_off(L);
+  double *stacks = f.stacks + (size_t) type * NG_COMMITTED * Ns;
+  double *stk = stacks + (size_t) kTermGrid[term] * Ns, *mstk = stacks + (size_t) GALIC_GRID_MASS_I * Ns;
+  const double *grids = f.committed + (size_t) type * NG_COMMITTED * f.Ngrid;
+  const double *fine = from_stacks ? stk + off : grids + (size_t) kTermGrid[term] * f.Ngrid;
+  const double *mfine = from_stacks ? mstk + off : grids + (size_t) GALIC_GRID_MASS_I * f.Ngrid;
+  double *val = f.values + ((size_t) type * NTERM + term) * Ns;
+  const TermLeaf<KIND> leaf(f, type, term);
+  auto children = [&](int g, double (&x)[1][4], double (&m)[4]) {
+    const int at[4] = {g, g + 1, g + N, g + N + 1};
+#pragma unroll
+    for(int q = 0; q < 4; q++) {
+      x[0][q] = fine[at[q]];
+      if(KIND == 2) m[q] = mfine[at[q]];
+    }
+    if(!from_stacks)
+#pragma unroll
+      for(int q = 0; q < 4; q++) {
+        stk[off + at[q]] = x[0][q];
+        if(KIND == 2 && term == 5) mstk[off + at[q]] = m[q];
+      }
+    return 1u;
+  };
+  auto keep = [&](int node, double d, double v, double r) {
+    val[node] = v;
+    if(!from_stacks) {
+      stk[node] = d;
+      if(KIND == 2 && term == 5) mstk[node] = r;
+    }
+  };
+  auto keep_leaf = [&](int node, double v) { val[node] = v; };
+  double root[1];
+  pyramid_cta<1, KIND == 2>(sm, L, children, [](int) { return 0.0; }, leaf,
+                            f.targets + ((size_t) type * NT_TARGET + T_DGM) * Ns, KIND == 2 ? f.thr_e[type] : f.thr_d[type],
+                            keep, keep_leaf, root);
+  return root[0];
 }
 
-__global__ void k_fit_final(FitArgs f, const double *raw)
+__device__ __forceinline__ void fit_final(const FitArgs &f, int type)
 {
-  const int type = threadIdx.x;
-  if(type < 1 || type > 3 || !f.present[type]) return;
+  const volatile double *raw = f.raw + type * 5;
   const double *tg = f.targets + (size_t) type * NT_TARGET * f.Nstack;
-  double S = raw[type * 5 + 0];
+  double S = raw[0];
   S *= 1.0 / tg[T_DGM * f.Nstack + 0];
-  double sr = raw[type * 5 + 1], st = raw[type * 5 + 2], sp = raw[type * 5 + 3], sq = raw[type * 5 + 4];
+  double sr = raw[1], st = raw[2], sp = raw[3], sq = raw[4];
   double count;
   if(f.tovs[type] == 0 || f.tovs[type] == 1) {
     count = 3.0;
@@ -102,6 +125,40 @@ __global__ void k_fit_final(FitArgs f, const double *raw)
   o[4] = sq * srel;
   o[5] = srel;
   o[6] = count;
+}
+
+// One CTA per (type, term): smooths the term's stack, evaluates its misfit and
+// leaves both, node by node (f.stacks, f.values); the CTA of a type that ends
+// last forms the type's fit.  The three kernels it replaces (smooth, misfit on
+// a whole stack in shared memory, final) took 32 us at level 6, with 21 us more
+// for the committed instantaneous terms; it takes 15 us (cold caches).
+__global__ void __launch_bounds__(1024) k_fit(const __grid_constant__ FitArgs f, int first, int count,
+                                              bool from_stacks, double *hist)
+{
+  __shared__ union {
+    Pyramid<1, false> a;
+    Pyramid<1, true> b;
+  } sm;
+  const int type = (int) blockIdx.x / count, term = first + (int) blockIdx.x % count;
+  if(type < 1 || !f.present[type]) {
+    if(hist && term == 0 && threadIdx.x < 7) hist[type * 7 + threadIdx.x] = f.fit[type * 7 + threadIdx.x];
+    return;
+  }
+  const double v = term == 0 ? fit_term<0>(f, type, term, from_stacks, sm.a)
+                             : (term < 5 ? fit_term<1>(f, type, term, from_stacks, sm.a)
+                                         : fit_term<2>(f, type, term, from_stacks, sm.b));
+  if(threadIdx.x || from_stacks) return;
+  // raw[type][w]: w = 0 S, 1 Sdisp_r, 2 Sdisp_t, 3 Sdisp_p, 4 Sdisp_q
+  if(term == 0 || term >= 5) {
+    *(volatile double *) &f.raw[type * 5 + (term ? term - 4 : 0)] = v;
+    __threadfence();
+    if(atomicInc(&f.arrived[type], 4) == 4) {  // (wraps to 0)
+      __threadfence();
+      fit_final(f, type);
+      if(hist)
+        for(int j = 0; j < 7; j++) hist[type * 7 + j] = f.fit[type * 7 + j];
+    }
+  }
 }
 
 // ---------------------------------------------------------------- optimize
@@ -151,6 +208,9 @@ __global__ void k_propose(DevModel M, RepArgs R)
     }
   } while(sqrt(v2_new) >= M.MaxVelInUnitsVesc * R.p_vesc[n]);
   if(st_code) atomicMax(R.status, st_code);
+  // what the trial would change in the energy grid (add_to_energy_grid)
+  disp_components(M, L, type, pos, v_new, &R.try_disp[4 * k]);
+  R.inst_cell[k] = energy_cell(M, L, pos);
   for(int j = 0; j < 3; j++) {
     R.vel_try[3 * k + j] = v_new[j];
     R.b_pos[3 * (2 * k) + j] = pos[j];
@@ -163,118 +223,130 @@ __global__ void k_propose(DevModel M, RepArgs R)
   R.b_type[2 * k] = R.b_type[2 * k + 1] = type;
 }
 
-// The nine stack terms of eval_fit_mod (main.c:1021-1217), one CTA per
-// (particle k, which, term): which 0 = F_base, 1 = F_try; term 0 the
-// density term (main.c:1033-1047), 1-4 the time-averaged dispersion terms
-// r, t, q, p (main.c:1052-1120), 5-8 the instantaneous terms r, t, p, q
-// (main.c:1125-1176).  Each writes its stack difference to
-// R.F[(2k + which) * NTERM + term]; k_accept combines them into F in the
-// reference's order.
-// The base evaluation's instantaneous terms (which 0, terms 5-8) are not
-// launched per particle: its velocity is the particle's own, whose
-// projections are the committed ones (p_vdisp was computed from p_vel by
-// the same disp_components), so the change it adds to the energy grid is
-// exactly zero and the term is its type's committed misfit, computed once
-// per repetition by k_base_inst.  Each particle launches 5 + 9 CTAs.
-enum { NTERM = 9, NLAUNCH = 14 };
+// The stack terms of eval_fit_mod, to R.F[(2k + which) * NTERM + term]; which
+// 0 = F_base, 1 = F_try.  What it needs is the old and trial orbits' grids once
+// (10 x 2^2L doubles per particle); what an orbit leaves as it was keeps its
+// committed value (f.values), so only the part of the grid that an orbit
+// crosses costs leaf terms with their divisions.  One CTA per particle and term
+// evaluates both sums from one read of the grids.
+//   The base evaluation's instantaneous terms are not evaluated per particle:
+// its velocity is the particle's own, whose projections are the committed ones
+// (p_vdisp was computed from p_vel by the same disp_components), so the change
+// it adds to the energy grid is exactly zero and the term is its type's
+// committed misfit (f.values' root).  The trial's instantaneous terms change
+// four finest nodes, at most four per level: four lanes climb the levels.
+// 101 particles at level 6: 103 -> 33 us (cold caches), beside 12 and 4 -> 9 us
+// for the acceptance and the list, 78 -> 14 us for the commit: a construction with
+// 100 such repetitions 54 -> 41.5 ms.
+constexpr int EVAL_BLOCK = 256;
 
-__global__ void __launch_bounds__(512) k_eval_terms(DevModel M, RepArgs R, FitArgs f)
+// the trial's instantaneous term a (0-3: r, t, p, q) of particle k, on four
+// neighbouring lanes: lane q = 2 dz + dR follows the corner (iz + dz, iR + dR)
+__device__ __forceinline__ void eval_inst_term(const RepArgs &R, const FitArgs &f, int k, int a, bool act)
 {
-  // levels 0 .. L-1 of the evaluated stack; its finest level is formed on
-  // the fly from the committed stack and the orbit grids (stack.cuh:*_from)
-  extern __shared__ double sm[];
-  __shared__ double sh_d[4];
-  __shared__ Cell sh_c;
-  const int j = blockIdx.x % NLAUNCH, k = blockIdx.x / NLAUNCH;
-  const int which = j < 5 ? 0 : 1, term = j < 5 ? j : j - 5;
-  const int n = R.idx[k];
-  const int type = R.p_type[n];
-  const int L = f.L, G = f.Ngrid, Ns = f.Nstack;
-  const int off = ((1 << (2 * L)) - 1) / 3;
-  const double *gold = R.grids + (size_t) (2 * k) * NF_ORBIT * G;
-  const double *gnew = R.grids + (size_t) (2 * k + which) * NF_ORBIT * G;
-  // the orbit grids are stored unscaled: x mass/tall on the fly, the
-  // operation k_scale_dense would have applied
-  const double fo = R.b_mass[2 * k] / R.b_tall[2 * k];
-  const double fn = R.b_mass[2 * k + which] / R.b_tall[2 * k + which];
-  const double *stk = f.stacks + (size_t) type * NG_COMMITTED * Ns;
-  const double *tg = f.targets + (size_t) type * NT_TARGET * Ns;
-  double v;
-  if(term == 0) {
-    // density term: committed + new - old
-    const double *c = stk + (size_t) GALIC_GRID_MASS_S * Ns + off;
-    const double *gn = gnew + F_M * G, *go = gold + F_M * G;
-    auto fin = [&](int i) { return c[i] + gn[i] * fn - go[i] * fo; };
-    stack_smooth_cta_from(sm, L, fin);
-    v = stack_diff_cta_from(sm, fin, tg + T_DGM * Ns, tg + T_DGM * Ns, nullptr, f.dgs_distance, f.thr_d[type], 0, 0,
-                            L, f.R200_20, f.LowerDispLimit);
-  } else if(term <= 4) {
-    // time-averaged dispersion terms r, t, q, p
-    const int a = term - 1;
-    const int fs[4] = {F_R, F_T, F_Q, F_P};
-    const int gs[4] = {GALIC_GRID_R_S, GALIC_GRID_T_S, GALIC_GRID_Q_S, GALIC_GRID_P_S};
-    const int ts[4] = {T_R, T_T, T_Q, T_P};
-    const double *c = stk + (size_t) gs[a] * Ns + off;
-    const double *gn = gnew + fs[a] * G, *go = gold + fs[a] * G;
-    auto fin = [&](int i) { return c[i] + gn[i] * fn - go[i] * fo; };
-    stack_smooth_cta_from(sm, L, fin);
-    v = stack_diff_cta_from(sm, fin, tg + ts[a] * Ns, tg + T_DGM * Ns, tg + ts[a] * Ns, f.dgs_distance,
-                            f.thr_d[type], 2, 1, L, f.R200_20, f.LowerDispLimit);
-  } else {
-    // instantaneous terms r, t, p, q of the trial velocity: its change of the
-    // particle's projections at its energy-grid cell
-    const int a = term - 5;
-    if(threadIdx.x == 0) {
-      LogConsts Lc = make_log_consts(M);
-      const double *vel = which ? &R.vel_try[3 * k] : &R.p_vel[3 * n];
-      disp_components(M, Lc, type, &R.p_pos[3 * n], vel, sh_d);
-      sh_c = energy_cell(M, Lc, &R.p_pos[3 * n]);
+  const int lane = threadIdx.x & 31, q = lane & 3, quad = lane & ~3;
+  const int n = R.idx[k], type = R.p_type[n];
+  const int L = f.L, Ns = f.Nstack;
+  const double *stk = f.stacks + ((size_t) type * NG_COMMITTED + kTermGrid[5 + a]) * Ns;
+  const double *ms = f.stacks + ((size_t) type * NG_COMMITTED + GALIC_GRID_MASS_I) * Ns;
+  const double *val = f.values + ((size_t) type * NTERM + 5 + a) * Ns;
+  const TermLeaf<2> leaf(f, type, 5 + a);
+  const double thr = f.thr_e[type];
+  // add_to_energy_grid: vr2 *= mass etc. (main.c:885-888); order r, t, p, q
+  const double dv = (R.try_disp[4 * k + a] - R.p_vdisp[4 * n + a]) * R.p_mass[n];
+  const Cell cc = R.inst_cell[k];
+  const double w = q == 0 ? (1 - cc.fR) * (1 - cc.fz)
+                          : (q == 1 ? (cc.fR) * (1 - cc.fz) : (q == 2 ? (1 - cc.fR) * (cc.fz) : (cc.fR) * (cc.fz)));
+  const int dz = q >> 1, dR = q & 1;
+  // the two rows and columns that the corners' nodes have at this level
+  int z0 = cc.iz, z1 = cc.iz + 1, r0 = cc.iR, r1 = cc.iR + 1;
+  int node = stack_off(L) + ((dz ? z1 : z0) << L) + (dR ? r1 : r0);
+  double d = stk[node] + w * dv;
+  double v = leaf(node, d, ms[node]);
+  for(int l = L - 1; l >= 0; l--) {
+    const int pz = (dz ? z1 : z0) >> 1, pr = (dR ? r1 : r0) >> 1, cn = 2 << l;
+    double cd[4], cv[4];
+#pragma unroll
+    for(int c = 0; c < 4; c++) {
+      const int z = 2 * pz + (c >> 1), r = 2 * pr + (c & 1), at = stack_off(l + 1) + z * cn + r;
+      const int iz = z == z0 ? 0 : (z == z1 ? 1 : -1), ir = r == r0 ? 0 : (r == r1 ? 1 : -1);
+      const int src = quad + (iz > 0 ? 2 : 0) + (ir > 0 ? 1 : 0);
+      const double sd = __shfl_sync(0xffffffffu, d, src), sv = __shfl_sync(0xffffffffu, v, src);
+      const bool own = iz >= 0 && ir >= 0;
+      cd[c] = own ? sd : stk[at];
+      cv[c] = own ? sv : val[at];
     }
-    __syncthreads();
-    const double mass = R.p_mass[n];
-    const double *vd = &R.p_vdisp[4 * n];
-    // add_to_energy_grid: vr2 *= mass etc. (main.c:885-888); order r, t, p, q
-    const double dv = (sh_d[a] - vd[a]) * mass;
-    const int gi[4] = {GALIC_GRID_R_I, GALIC_GRID_T_I, GALIC_GRID_P_I, GALIC_GRID_Q_I};
-    const int ti[4] = {T_R, T_T, T_P, T_Q};
-    const Cell cc = sh_c;
-    const int Nb = 1 << L;
-    const int c00 = cc.iz * Nb + cc.iR;
-    const double w00 = (1 - cc.fR) * (1 - cc.fz), w10 = (cc.fR) * (1 - cc.fz), w01 = (1 - cc.fR) * (cc.fz),
-                 w11 = (cc.fR) * (cc.fz);
-    const double *c = stk + (size_t) gi[a] * Ns + off;
-    // committed value, plus w * dv at the four corners of the cell
-    auto fin = [&](int i) {
-      const double x = c[i];
-      return i == c00 ? x + w00 * dv
-                      : (i == c00 + 1 ? x + w10 * dv : (i == c00 + Nb ? x + w01 * dv : (i == c00 + Nb + 1 ? x + w11 * dv : x)));
-    };
-    stack_smooth_cta_from(sm, L, fin);
-    v = stack_diff_cta_from(sm, fin, tg + ti[a] * Ns, stk + (size_t) GALIC_GRID_MASS_I * Ns, tg + T_EGM * Ns,
-                            nullptr, f.thr_e[type], 1, 0, L, f.R200_20, f.LowerDispLimit);
+    node = stack_off(l) + (pz << l) + pr;
+    const double m = ms[node];
+    d = cd[0] + cd[2] + cd[1] + cd[3];
+    if(m < thr) {
+      v = leaf(node, d, m);
+    } else {
+      v = cv[0];
+      v += cv[1];
+      v += cv[2];
+      v += cv[3];
+    }
+    z0 >>= 1, z1 >>= 1, r0 >>= 1, r1 >>= 1;
   }
-  if(threadIdx.x == 0) R.F[(2 * k + which) * NTERM + term] = v;
+  if(act && q == 0) R.F[(2 * k + 1) * NTERM + 5 + a] = v;
 }
 
-// the committed instantaneous misfit of each present type: terms 5-8 of
-// every base evaluation of the repetition (see k_eval_terms)
-__global__ void __launch_bounds__(512) k_base_inst(RepArgs R, FitArgs f)
+template <int KIND>
+__device__ __forceinline__ void eval_orbit_term(const RepArgs &R, const FitArgs &f, int k, int term,
+                                                Pyramid<2, false> &sm)
 {
-  extern __shared__ double sm[];
-  const int type = blockIdx.x >> 2, a = blockIdx.x & 3;
-  if(type < 1 || !f.present[type]) return;
-  const int L = f.L, Ns = f.Nstack;
-  const int off = ((1 << (2 * L)) - 1) / 3;
-  const double *stk = f.stacks + (size_t) type * NG_COMMITTED * Ns;
-  const double *tg = f.targets + (size_t) type * NT_TARGET * Ns;
-  const int gi[4] = {GALIC_GRID_R_I, GALIC_GRID_T_I, GALIC_GRID_P_I, GALIC_GRID_Q_I};
-  const int ti[4] = {T_R, T_T, T_P, T_Q};
-  const double *c = stk + (size_t) gi[a] * Ns + off;
-  auto fin = [&](int i) { return c[i]; };
-  stack_smooth_cta_from(sm, L, fin);
-  const double v = stack_diff_cta_from(sm, fin, tg + ti[a] * Ns, stk + (size_t) GALIC_GRID_MASS_I * Ns,
-                                       tg + T_EGM * Ns, nullptr, f.thr_e[type], 1, 0, L, f.R200_20, f.LowerDispLimit);
-  if(threadIdx.x == 0) R.inst0[blockIdx.x] = v;
+  const int n = R.idx[k], type = R.p_type[n];
+  const int L = f.L, N = 1 << L, G = f.Ngrid, Ns = f.Nstack;
+  // orbit fields m, r, t, q, p, as the terms
+  const double *gold = R.grids + ((size_t) (2 * k) * NF_ORBIT + term) * G;
+  const double *gnew = gold + (size_t) NF_ORBIT * G;
+  // the orbit grids are stored unscaled: x mass/tall on the fly, the
+  // operation k_scale_dense would have applied
+  const double fo = R.b_mass[2 * k] / R.b_tall[2 * k], fn = R.b_mass[2 * k + 1] / R.b_tall[2 * k + 1];
+  const double *c = f.stacks + ((size_t) type * NG_COMMITTED + kTermGrid[term]) * Ns + stack_off(L);
+  const double *val = f.values + ((size_t) type * NTERM + term) * Ns;
+  const TermLeaf<KIND> leaf(f, type, term);
+  // committed + new - old
+  auto children = [&](int g, double (&x)[2][4], double (&)[4]) {
+    unsigned changed = 0;
+#pragma unroll
+    for(int z = 0; z < 2; z++) {
+      const double2 o = *(const double2 *) &gold[g + z * N], w = *(const double2 *) &gnew[g + z * N];
+      const double c0 = c[g + z * N], c1 = c[g + z * N + 1];
+      x[0][2 * z] = c0 + o.x * fo - o.x * fo;
+      x[0][2 * z + 1] = c1 + o.y * fo - o.y * fo;
+      x[1][2 * z] = c0 + w.x * fn - o.x * fo;
+      x[1][2 * z + 1] = c1 + w.y * fn - o.y * fo;
+      changed |= (x[0][2 * z] != c0 || x[0][2 * z + 1] != c1 ? 1u : 0u) |
+                 (x[1][2 * z] != c0 || x[1][2 * z + 1] != c1 ? 2u : 0u);
+    }
+    return changed;
+  };
+  double root[2];
+  pyramid_cta<2, false>(sm, L, children, [&](int node) { return val[node]; }, leaf,
+                        f.targets + ((size_t) type * NT_TARGET + T_DGM) * Ns, f.thr_d[type],
+                        [](int, double, double, double) {}, [](int, double) {}, root);
+  if(threadIdx.x == 0) {
+    R.F[(2 * k) * NTERM + term] = root[0];
+    R.F[(2 * k + 1) * NTERM + term] = root[1];
+  }
+}
+
+// the first inst_blocks CTAs: the instantaneous terms
+__global__ void __launch_bounds__(EVAL_BLOCK, 3)
+    k_eval_terms(const __grid_constant__ RepArgs R, const __grid_constant__ FitArgs f, int inst_blocks)
+{
+  __shared__ Pyramid<2, false> sm;
+  if((int) blockIdx.x < inst_blocks) {
+    const int item = (int) (blockIdx.x * (EVAL_BLOCK / 4) + (threadIdx.x >> 2));
+    const bool act = item < 4 * R.count;
+    eval_inst_term(R, f, act ? item >> 2 : 0, act ? item & 3 : 0, act);
+    return;
+  }
+  const int j = (int) blockIdx.x - inst_blocks, k = j / 5, term = j % 5;
+  if(term == 0) eval_orbit_term<0>(R, f, k, term, sm);
+  else eval_orbit_term<1>(R, f, k, term, sm);
 }
 
 // F of eval_fit_mod from its nine stack terms t[] (main.c:1047, 1120, 1195-1212)
@@ -294,159 +366,166 @@ __device__ __forceinline__ double combine_terms(const DevModel &M, const RepArgs
              4;
 }
 
-__global__ void k_accept(DevModel M, RepArgs R, FitArgs f)
+// Accepts and lists the accepted positions of each type in increasing order
+// (one CTA, in rounds of its threads); k_commit loops over these instead of over
+// every position.
+__global__ void __launch_bounds__(1024) k_accept(const __grid_constant__ DevModel M, const __grid_constant__ RepArgs R,
+                                                 const __grid_constant__ FitArgs f)
 {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if(k >= R.count) return;
-  const int n = R.idx[k];
-  const int type = R.p_type[n];
-  R.p_orbits[n] = R.b_norbit[2 * k];  // main.c:460 writes the old orbit's count
-  atomicAdd(&R.tries[type], 1ULL);
-  double tb[NTERM];
-  for(int j = 0; j < 5; j++) tb[j] = R.F[(2 * k) * NTERM + j];
-  for(int j = 0; j < 4; j++) tb[5 + j] = R.inst0[4 * type + j];
-  const double F_base = combine_terms(M, R, f, type, tb);
-  const double F_try = combine_terms(M, R, f, type, &R.F[(2 * k + 1) * NTERM]);
-  const bool acc = F_try < F_base;  // main.c:468
-  // mass/tall of the old and trial orbits (orbit_response.c:477-486) for
-  // the commit, which reads the unscaled orbit grids
-  R.fac[2 * k] = R.b_mass[2 * k] / R.b_tall[2 * k];
-  R.fac[2 * k + 1] = R.b_mass[2 * k + 1] / R.b_tall[2 * k + 1];
-  R.accepted[k] = acc ? 1 : 0;
-  if(!acc) return;
-  for(int j = 0; j < 3; j++) R.p_vel[3 * n + j] = R.vel_try[3 * k + j];
-  R.p_orbits[n] = R.b_norbit[2 * k + 1];
-  atomicAdd(&R.changes[type], 1ULL);
-  LogConsts L = make_log_consts(M);
-  double d[4];
-  disp_components(M, L, type, &R.p_pos[3 * n], &R.vel_try[3 * k], d);
-  double *vd = &R.p_vdisp[4 * n];
-  const double mass = R.p_mass[n];
-  for(int j = 0; j < 4; j++) {
-    R.inst_v[4 * k + j] = (d[j] - vd[j]) * mass;
-    vd[j] = d[j];
-  }
-  R.inst_cell[k] = energy_cell(M, L, &R.p_pos[3 * n]);
-}
-
-// the accepted positions of one repetition in increasing k (one CTA): the
-// commit kernels below loop over these instead of over every position
-__global__ void __launch_bounds__(1024) k_compact(RepArgs R)
-{
-  __shared__ int warp_sum[32];
-  __shared__ int base;
+  __shared__ int warp_sum[3][32];
+  int listed[3] = {0, 0, 0};  // accepted so far, types 1 to 3
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if(threadIdx.x == 0) base = 0;
-  __syncthreads();
   for(int k0 = 0; k0 < R.count; k0 += blockDim.x) {
     const int k = k0 + threadIdx.x;
-    const int a = (k < R.count && R.accepted[k]) ? 1 : 0;
-    const unsigned m = __ballot_sync(0xffffffffu, a);
-    if(lane == 0) warp_sum[wid] = __popc(m);
+    const bool act = k < R.count;
+    int type = 0;
+    bool acc = false;
+    if(act) {
+      const int n = R.idx[k];
+      type = R.p_type[n];
+      double tb[NTERM];
+      for(int j = 0; j < 5; j++) tb[j] = R.F[(2 * k) * NTERM + j];
+      for(int j = 0; j < 4; j++) tb[5 + j] = f.values[((size_t) type * NTERM + 5 + j) * f.Nstack];
+      const double F_base = combine_terms(M, R, f, type, tb);
+      const double F_try = combine_terms(M, R, f, type, &R.F[(2 * k + 1) * NTERM]);
+      acc = F_try < F_base;  // main.c:468
+      // mass/tall of the old and trial orbits (orbit_response.c:477-486) for
+      // the commit, which reads the unscaled orbit grids
+      R.fac[2 * k] = R.b_mass[2 * k] / R.b_tall[2 * k];
+      R.fac[2 * k + 1] = R.b_mass[2 * k + 1] / R.b_tall[2 * k + 1];
+      R.p_orbits[n] = R.b_norbit[2 * k + (acc ? 1 : 0)];  // main.c:460 writes the old orbit's count
+      if(acc) {
+        for(int j = 0; j < 3; j++) R.p_vel[3 * n + j] = R.vel_try[3 * k + j];
+        double *vd = &R.p_vdisp[4 * n];
+        const double mass = R.p_mass[n];
+        for(int j = 0; j < 4; j++) {
+          const double d = R.try_disp[4 * k + j];
+          R.inst_v[4 * k + j] = (d - vd[j]) * mass;
+          vd[j] = d;
+        }
+      }
+    }
+    int before[3];
+#pragma unroll
+    for(int t = 0; t < 3; t++) {
+      const unsigned tried = __ballot_sync(0xffffffffu, act && type == t + 1),
+                     m = __ballot_sync(0xffffffffu, acc && type == t + 1);
+      before[t] = __popc(m & ((1u << lane) - 1));
+      if(lane == 0) {
+        warp_sum[t][wid] = __popc(m);
+        if(tried) atomicAdd(&R.tries[t + 1], (unsigned long long) __popc(tried));
+        if(m) atomicAdd(&R.changes[t + 1], (unsigned long long) __popc(m));
+      }
+    }
     __syncthreads();
-    int before = 0;
-    for(int w = 0; w < wid; w++) before += warp_sum[w];
-    if(a) R.acc_list[base + before + __popc(m & ((1u << lane) - 1))] = k;
-    __syncthreads();
-    if(threadIdx.x == 0) {
-      int tot = 0;
-      for(int w = 0; w < (int) (blockDim.x >> 5); w++) tot += warp_sum[w];
-      base += tot;
+#pragma unroll
+    for(int t = 0; t < 3; t++) {
+      int at = listed[t] + before[t];
+      for(int w = 0; w < (int) (blockDim.x >> 5); w++) {
+        if(w < wid) at += warp_sum[t][w];
+        listed[t] += warp_sum[t][w];
+      }
+      if(acc && type == t + 1) R.acc_list[(size_t) t * R.count + at] = k;
     }
     __syncthreads();
   }
-  if(threadIdx.x == 0) *R.acc_n = base;
+  if(threadIdx.x < 3) R.acc_n[threadIdx.x] = listed[threadIdx.x];
 }
 
-// per (type, field, bin): delta = sum over accepted particles, in order, of
-// new - old; committed += delta
-__global__ void k_delta_cols(RepArgs R, FitArgs f)
-{
-  const int G = f.Ngrid;
-  const int na = *R.acc_n;
-  const size_t total = (size_t) 4 * NF_ORBIT * G;
-  for(size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x; t < total; t += (size_t) gridDim.x * blockDim.x) {
-    const int type = (int) (t / ((size_t) NF_ORBIT * G));
-    const int fld = (int) ((t / G) % NF_ORBIT);
-    const int i = (int) (t % G);
-    if(type < 1 || !f.present[type]) continue;
-    double delta = 0;
-    for(int j = 0; j < na; j++) {
-      const int k = R.acc_list[j];
-      if(R.b_type[2 * k] != type) continue;
-      const double *gold = R.grids + (size_t) (2 * k) * NF_ORBIT * G;
-      const double *gnew = gold + (size_t) NF_ORBIT * G;
-      // unscaled orbit grids: x mass/tall as k_scale_dense would (the
-      // factors k_accept stored, the same divisions)
-      delta += gnew[fld * G + i] * R.fac[2 * k + 1] - gold[fld * G + i] * R.fac[2 * k];
-    }
-    // orbit fields m,r,t,q,p map to committed MASS_S, R_S, T_S, Q_S, P_S
-    double *dst = (double *) f.committed + ((size_t) type * NG_COMMITTED + fld) * G + i;
-    *dst += delta;
-  }
-}
+// Adds the accepted particles' changes to the committed grids, one thread per
+// bin.  blockIdx.y = 6 (type - 1) + field: fields 0 to 4 the orbits', new - old;
+// 5 the energy grid's four.  A thread's sum is a chain in particle order, so
+// the accepted list is staged in shared memory and eight particles' values are
+// on their way at a time (the grids were read once by the evaluation and mostly
+// come from L2).
+constexpr int COMMIT_BLOCK = 128, COMMIT_LIST = 256;
 
-__global__ void k_inst_delta(RepArgs R, FitArgs f)
+__global__ void __launch_bounds__(COMMIT_BLOCK) k_commit(const __grid_constant__ RepArgs R,
+                                                         const __grid_constant__ FitArgs f)
 {
+  __shared__ int s_k[COMMIT_LIST];
+  __shared__ double s_a[COMMIT_LIST], s_b[COMMIT_LIST];
+  __shared__ double s_v[COMMIT_LIST][4];
+  const int type = blockIdx.y / 6 + 1, fld = blockIdx.y % 6;
+  if(!f.present[type]) return;
   const int G = f.Ngrid, Nb = 1 << f.L;
-  const int na = *R.acc_n;
-  const size_t total = (size_t) 4 * 4 * G;
-  const int gi[4] = {GALIC_GRID_R_I, GALIC_GRID_T_I, GALIC_GRID_P_I, GALIC_GRID_Q_I};
-  for(size_t t = blockIdx.x * (size_t) blockDim.x + threadIdx.x; t < total; t += (size_t) gridDim.x * blockDim.x) {
-    const int type = (int) (t / ((size_t) 4 * G));
-    const int a = (int) ((t / G) % 4);
-    const int cidx = (int) (t % G);
-    if(type < 1 || !f.present[type]) continue;
-    double delta = 0;
-    for(int j = 0; j < na; j++) {
-      const int k = R.acc_list[j];
-      if(R.b_type[2 * k] != type) continue;
-      const Cell c = R.inst_cell[k];
-      const int base = c.iz * Nb + c.iR;
-      double w;
-      if(cidx == base) w = (1 - c.fR) * (1 - c.fz);
-      else if(cidx == base + 1) w = (c.fR) * (1 - c.fz);
-      else if(cidx == base + Nb) w = (1 - c.fR) * (c.fz);
-      else if(cidx == base + Nb + 1) w = (c.fR) * (c.fz);
-      else continue;
-      // inst_v holds (vr2, vt2, vp2, vq2) differences times mass
-      delta += w * R.inst_v[4 * k + a];
+  const int na = R.acc_n[type - 1];
+  const int *list = R.acc_list + (size_t) (type - 1) * R.count;
+  const int i = blockIdx.x * COMMIT_BLOCK + threadIdx.x;
+  double *dst = (double *) f.committed + (size_t) type * NG_COMMITTED * G + i;
+  double delta[4] = {0, 0, 0, 0};
+  for(int j0 = 0; j0 < na; j0 += COMMIT_LIST) {
+    const int nj = min(COMMIT_LIST, na - j0);
+    __syncthreads();
+    for(int j = threadIdx.x; j < nj; j += COMMIT_BLOCK) {
+      const int k = list[j0 + j];
+      if(fld < 5) {
+        // unscaled orbit grids: x mass/tall as k_scale_dense would (the
+        // factors k_accept stored, the same divisions)
+        s_k[j] = k;
+        s_a[j] = R.fac[2 * k];
+        s_b[j] = R.fac[2 * k + 1];
+      } else {
+        const Cell c = R.inst_cell[k];
+        s_k[j] = c.iz * Nb + c.iR;
+        s_a[j] = c.fR;
+        s_b[j] = c.fz;
+        // inst_v holds (vr2, vt2, vp2, vq2) differences times mass
+        for(int a = 0; a < 4; a++) s_v[j][a] = R.inst_v[4 * k + a];
+      }
     }
-    double *dst = (double *) f.committed + ((size_t) type * NG_COMMITTED + gi[a]) * G + cidx;
-    *dst += delta;
+    __syncthreads();
+    if(i >= G) continue;
+    if(fld < 5) {
+      const double *base = R.grids + (size_t) fld * G + i;
+      const size_t orbit = (size_t) NF_ORBIT * G;
+      int j = 0;
+      for(; j + 8 <= nj; j += 8) {
+        double o[8], w[8];
+#pragma unroll
+        for(int u = 0; u < 8; u++) {
+          const double *g = base + (size_t) (2 * s_k[j + u]) * orbit;
+          o[u] = g[0];
+          w[u] = g[orbit];
+        }
+#pragma unroll
+        for(int u = 0; u < 8; u++) delta[0] += w[u] * s_b[j + u] - o[u] * s_a[j + u];
+      }
+      for(; j < nj; j++) {
+        const double *g = base + (size_t) (2 * s_k[j]) * orbit;
+        delta[0] += g[orbit] * s_b[j] - g[0] * s_a[j];
+      }
+    } else {
+      for(int j = 0; j < nj; j++) {
+        const int at = i - s_k[j];
+        const double fR = s_a[j], fz = s_b[j];
+        double w;
+        if(at == 0) w = (1 - fR) * (1 - fz);
+        else if(at == 1) w = (fR) * (1 - fz);
+        else if(at == Nb) w = (1 - fR) * (fz);
+        else if(at == Nb + 1) w = (fR) * (fz);
+        else continue;
+#pragma unroll
+        for(int a = 0; a < 4; a++) delta[a] += w * s_v[j][a];
+      }
+    }
+  }
+  if(i >= G) return;
+  if(fld < 5) {
+    // orbit fields m,r,t,q,p map to committed MASS_S, R_S, T_S, Q_S, P_S
+    dst[(size_t) fld * G] += delta[0];
+  } else {
+#pragma unroll
+    for(int a = 0; a < 4; a++) dst[(size_t) kTermGrid[5 + a] * G] += delta[a];
   }
 }
 
 }  // namespace
 
-// the stack kernels keep a whole level-7 stack (171 KiB) in shared memory;
-// called once per context, on the context's device
-// the shared-memory opt-in of the stack kernels, once per device
-cudaError_t prepare_fit_kernels()
+int launch_global_fit(const FitArgs &f, cudaStream_t s, double *hist, int first, int count)
 {
-  static std::mutex mu;
-  static bool done[256] = {false};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if(e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lk(mu);
-  if(dev >= 0 && dev < 256 && done[dev]) return cudaSuccess;
-  if((e = cudaFuncSetAttribute(k_fit_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024))) return e;
-  if((e = cudaFuncSetAttribute(k_fit_diff, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024))) return e;
-  if((e = cudaFuncSetAttribute(k_eval_terms, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024))) return e;
-  if((e = cudaFuncSetAttribute(k_base_inst, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024))) return e;
-  if(dev >= 0 && dev < 256) done[dev] = true;
-  return cudaSuccess;
-}
-
-int launch_global_fit(const FitArgs &f, cudaStream_t s)
-{
-  size_t smem = (size_t) f.Nstack * sizeof(double);
-  double *raw = f.fit + 4 * 7;  // scratch after the 4x7 fit block
-  k_fit_smooth<<<4 * NG_COMMITTED, 1024, smem, s>>>(f);
-  k_fit_diff<<<4 * 5, 1024, smem, s>>>(f, raw);
-  k_fit_final<<<1, 4, 0, s>>>(f, raw);
-  return 3;
+  k_fit<<<4 * count, 1024, 0, s>>>(f, first, count, false, hist);
+  return 1;
 }
 
 int launch_rep_orbits(const DevModel &M, const RepArgs &R, const OrbitBatch &b, cudaStream_t s,
@@ -464,19 +543,19 @@ int launch_rep_orbits(const DevModel &M, const RepArgs &R, const OrbitBatch &b, 
   return 2;
 }
 
-int launch_rep_commit(const DevModel &M, const RepArgs &R, const FitArgs &f, cudaStream_t s)
+int launch_rep_values(const FitArgs &f, cudaStream_t s)
 {
-  const int count = R.count;
-  // levels 0 .. L-1 of a stack in shared memory (43 KiB at L = 7): four
-  // CTAs of 512 threads per SM
-  const size_t smem = (size_t) (((1 << (2 * f.L)) - 1) / 3) * sizeof(double);
-  k_base_inst<<<16, 512, smem, s>>>(R, f);
-  k_eval_terms<<<count * NLAUNCH, 512, smem, s>>>(M, R, f);
-  k_accept<<<(count + 127) / 128, 128, 0, s>>>(M, R, f);
-  k_compact<<<1, 1024, 0, s>>>(R);
-  k_delta_cols<<<148 * 8, 256, 0, s>>>(R, f);
-  k_inst_delta<<<148 * 8, 256, 0, s>>>(R, f);
-  return 6 + launch_global_fit(f, s);
+  k_fit<<<4 * NTERM, 1024, 0, s>>>(f, 0, NTERM, true, nullptr);
+  return 1;
+}
+
+int launch_rep_commit(const DevModel &M, const RepArgs &R, const FitArgs &f, cudaStream_t s, double *hist)
+{
+  const int count = R.count, inst_blocks = (4 * count + EVAL_BLOCK / 4 - 1) / (EVAL_BLOCK / 4);
+  k_eval_terms<<<inst_blocks + 5 * count, EVAL_BLOCK, 0, s>>>(R, f, inst_blocks);
+  k_accept<<<1, count < 1024 ? (count + 31) / 32 * 32 : 1024, 0, s>>>(M, R, f);
+  k_commit<<<dim3((f.Ngrid + COMMIT_BLOCK - 1) / COMMIT_BLOCK, 18), COMMIT_BLOCK, 0, s>>>(R, f);
+  return 3 + launch_global_fit(f, s, hist);
 }
 
 RepArgs rep_slice(const RepArgs &R, int first, int count, int G)
@@ -496,9 +575,9 @@ RepArgs rep_slice(const RepArgs &R, int first, int count, int G)
   S.grids = R.grids + (size_t) (2 * first) * NF_ORBIT * G;
   S.vel_try = R.vel_try + 3 * (size_t) first;
   S.F = R.F + 2 * (size_t) NTERM * first;
-  S.accepted = R.accepted + first;
-  S.acc_list = R.acc_list + first;
-  S.acc_n = R.acc_n + first / count;
+  S.acc_list = R.acc_list + 3 * (size_t) first;
+  S.acc_n = R.acc_n + 3 * (size_t) (first / count);
+  S.try_disp = R.try_disp + 4 * (size_t) first;
   S.inst_v = R.inst_v + 4 * (size_t) first;
   S.inst_cell = R.inst_cell + first;
   return S;
@@ -508,5 +587,5 @@ int launch_rep(const DevModel &M, const RepArgs &R, const FitArgs &f, const Orbi
                const float4 *const *quad32, const float *cellsize32)
 {
   const int launches = launch_rep_orbits(M, R, b, s, quad32, cellsize32);
-  return launches + launch_rep_commit(M, R, f, s);
+  return launches + launch_rep_values(f, s) + launch_rep_commit(M, R, f, s, nullptr);
 }

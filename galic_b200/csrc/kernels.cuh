@@ -62,14 +62,19 @@ struct CalcAllArgs {
   int *status;                // worst OrbitStatus seen
 };
 
+constexpr int FIT_TERMS = 9;
+
 struct FitArgs {
   int L;                      // DG_MaxLevel == EG_MaxLevel
   int Ngrid, Nstack;
   const double *committed;    // [4][10][Ngrid]
   double *stacks;             // [4][10][Nstack]
+  double *values;             // [4][9][Nstack]: node values of the committed merit terms (fit_fp64.cu:k_fit)
   const double *targets;      // [4][6][Nstack]
   const double *dgs_distance; // [Nstack]
   double *fit;                // [4][7]
+  double *raw;                // [4][5]
+  unsigned *arrived;          // [4], 0 between launches
   int *firstrun;              // [4]
   double thr_d[4], thr_e[4], MType[4];
   int present[4], tovs[4];
@@ -86,10 +91,12 @@ int launch_calc_all_fp64(const DevModel &M, const CalcAllArgs &a, int grid, int 
 void launch_instantaneous(const DevModel &M, int n, const double *pos, const double *vel, const double *mass,
                           const int *type, double *vdisp, FxWord *fx, const int *shift, int Ngrid, cudaStream_t s,
                           int first = 0, int stride = 1);
-void launch_fx_finalize(const FxWord *fx, const int *shift, double *committed, int count, int Ngrid, int form,
-                        cudaStream_t s);
-int launch_global_fit(const FitArgs &f, cudaStream_t s);
-cudaError_t prepare_fit_kernels();
+// grids first .. first + per - 1 of each of `sets` sets of NG_COMMITTED
+void launch_fx_finalize(const FxWord *fx, const int *shift, double *committed, int sets, int first, int per, int Ngrid,
+                        int form, cudaStream_t s);
+// hist: a second place for the fit ([4][7]), or null; terms first .. first +
+// count - 1 of FIT_TERMS only: the fit follows with the launch that completes them
+int launch_global_fit(const FitArgs &f, cudaStream_t s, double *hist = nullptr, int first = 0, int count = FIT_TERMS);
 int calc_all_occupancy(int block);
 int calc_all_fp32_occupancy(int block);
 int launch_calc_all_fp32(const DevModel &M64, const float4 *const quad[4], const float *cellsize32,

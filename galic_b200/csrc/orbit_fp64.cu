@@ -341,15 +341,18 @@ __global__ void k_instantaneous(DevModel M, int n, int first, int stride, const 
 
 // The time-averaged half of every set holds FxNode words (one_word: the FP32
 // form's single words), the instantaneous half word pairs grid by grid.
-__global__ void k_fx_finalize(const FxWord *fx, const int *shift, double *out, int count, int Ngrid, bool one_word)
+// The grids first .. first + per - 1 of each of the sets.
+__global__ void k_fx_finalize(const FxWord *fx, const int *shift, double *out, int sets, int first, int per, int Ngrid,
+                              bool one_word)
 {
-  size_t total = (size_t) count * Ngrid;
-  for(size_t i = blockIdx.x * (size_t) blockDim.x + threadIdx.x; i < total; i += (size_t) gridDim.x * blockDim.x) {
-    const int g = (int) (i / Ngrid), f = g % NG_COMMITTED;
+  const size_t total = (size_t) sets * per * Ngrid;
+  for(size_t j = blockIdx.x * (size_t) blockDim.x + threadIdx.x; j < total; j += (size_t) gridDim.x * blockDim.x) {
+    const int set = (int) (j / Ngrid) / per, f = first + (int) (j / Ngrid) % per, g = set * NG_COMMITTED + f;
+    const size_t i = (size_t) g * Ngrid + j % Ngrid;
     FxWord w;
     if(f < NF_ORBIT) {
       // (a set's first five grids are half of its NG_COMMITTED)
-      const FxNode *n = (const FxNode *) fx + (size_t) (g / NG_COMMITTED) * 2 * Ngrid + i % Ngrid;
+      const FxNode *n = (const FxNode *) fx + (size_t) set * 2 * Ngrid + j % Ngrid;
       w.hi = n->hi[f];
       w.lo = one_word ? 0 : n->lo[f];
     } else
@@ -398,11 +401,11 @@ void launch_instantaneous(const DevModel &M, int n, const double *pos, const dou
                                                       Ngrid);
 }
 
-void launch_fx_finalize(const FxWord *fx, const int *shift, double *committed, int count, int Ngrid, int form,
-                        cudaStream_t s)
+void launch_fx_finalize(const FxWord *fx, const int *shift, double *committed, int sets, int first, int per, int Ngrid,
+                        int form, cudaStream_t s)
 {
-  size_t total = (size_t) count * Ngrid;
+  size_t total = (size_t) sets * per * Ngrid;
   int grid = (int) ((total + 255) / 256);
   if(grid > 148 * 8) grid = 148 * 8;
-  k_fx_finalize<<<grid, 256, 0, s>>>(fx, shift, committed, count, Ngrid, form == GALIC_FORM_FP32);
+  k_fx_finalize<<<grid, 256, 0, s>>>(fx, shift, committed, sets, first, per, Ngrid, form == GALIC_FORM_FP32);
 }

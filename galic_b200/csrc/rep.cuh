@@ -29,12 +29,11 @@ struct RepArgs {
   double *fac;           // 2*count: mass / tall of each orbit (k_accept, for the commit)
   double *vel_try;  // count x 3
   double *F;        // 2*count x 9: the stack terms of F_base, F_try (fit_fp64.cu:k_eval_terms)
-  double *inst0;    // [4 types][4]: the committed instantaneous terms of the base evaluations
-  int *accepted;    // count
-  int *acc_list;    // count: the accepted positions k in increasing order (k_compact)
-  int *acc_n;       // one per repetition of the window: the length of its acc_list
+  double *try_disp; // count x 4: the trial velocity's projections (k_propose)
+  int *acc_list;    // 3 x count: the accepted positions k of types 1 to 3 in increasing order (k_accept)
+  int *acc_n;       // 3 per repetition of the window: their numbers
   double *inst_v;   // count x 4
-  Cell *inst_cell;  // count
+  Cell *inst_cell;  // count: the particles' energy-grid cells (k_propose)
   unsigned long long *tries, *changes;  // [4]
   double fac_rs[4], fac_ts[4], fac_qs[4], fac_ps[4];
   int *status;
@@ -48,7 +47,12 @@ int launch_rep(const DevModel &M, const RepArgs &R, const FitArgs &f, const Orbi
 // evaluation, acceptance and commit of ONE repetition whose arrays R points at
 int launch_rep_orbits(const DevModel &M, const RepArgs &R, const OrbitBatch &b, cudaStream_t s,
                       const float4 *const *quad32 = nullptr, const float *cellsize32 = nullptr);
-int launch_rep_commit(const DevModel &M, const RepArgs &R, const FitArgs &f, cudaStream_t s);
+// (hist: where the fit after it is stored as well, [4][7], or null).  The
+// repetitions of one call are preceded by launch_rep_values.
+int launch_rep_commit(const DevModel &M, const RepArgs &R, const FitArgs &f, cudaStream_t s, double *hist);
+// the node values of the committed terms (FitArgs::values) from the stacks, for
+// the first repetition of a call; each commit leaves the next one's
+int launch_rep_values(const FitArgs &f, cudaStream_t s);
 // R restricted to the `count` particles of window positions first ..
 // first + count - 1 (G: bins per grid)
 RepArgs rep_slice(const RepArgs &R, int first, int count, int G);

@@ -122,3 +122,63 @@ def test_windows_report_the_fit_after_every_repetition():
         got = ctx.optimize_reps(lists, 3, 10, window_bytes=4 * 60 * 2 * 5 * 1024 * 8 + 1, fits=True)
     assert got.shape == (len(lists), 4, 7)
     assert np.array_equal(got, np.stack(want), equal_nan=True)
+
+
+def misfit(d1, d2, r1, r2, level, thresh, low):
+    """calc_stack_difference with flag 1 (grid.c:1086-1151) of finest grids, bottom up."""
+    def children(a):
+        return a[0::2, 0::2], a[0::2, 1::2], a[1::2, 0::2], a[1::2, 1::2]
+
+    def leaf(d1, d2, r1, r2):
+        with np.errstate(all="ignore"):
+            q2 = d2 / r2
+            v = np.abs(d1 / r1 - q2) / np.where(q2 > low, q2, low)
+        return np.where((r1 > 0) & (r2 > 0), v, 0.0)
+
+    off = lambda l: (4 ** l - 1) // 3
+    at = lambda stack, l: stack[off(l):off(l + 1)].reshape(2 ** l, 2 ** l)
+    v = leaf(d1, at(d2, level), r1, at(r2, level))
+    for l in range(level - 1, -1, -1):
+        c = [children(x) for x in (d1, r1)]
+        d1, r1 = [((x[0] + x[2]) + x[1]) + x[3] for x in c]
+        x = children(v)
+        v = np.where(r1 < thresh, leaf(d1, at(d2, l), r1, at(r2, l)), ((x[0] + x[1]) + x[2]) + x[3])
+    return float(v[0, 0])
+
+
+@pytest.mark.parametrize("level", [1, 2, 3, 4, 5, 7])
+def test_fit_at_every_depth_of_the_pyramid(level):
+    """The merit takes the lowest three levels by shuffles and the rest through
+    shared memory: the instantaneous terms of the committed grids restated here, at
+    depths where one or the other is missing, and repetitions as single calls and
+    as windows."""
+    from galic_b200 import sampling
+    m = synth.config_composite(n_halo=300, n_disk=150, n_bulge=100, level=level, seed=57)
+    p = m.params
+    N = 2 ** level
+    with Context(p) as ctx:
+        states = []
+        lists = np.arange(540, dtype=np.int32).reshape(6, 90)
+        for windows in (False, True):
+            ctx.load_model(m)
+            ctx.calc_all_response_fields(GALIC_FORM_FP64)
+            if windows:
+                hist = ctx.optimize_reps(lists, 11, 70, GALIC_FORM_FP64, fits=True)
+            else:
+                each = []
+                for r in range(len(lists)):
+                    ctx.optimize_rep(lists[r], 11, 70 + r)
+                    each.append(ctx.fit())
+            states.append(state(ctx, (1, 2, 3))[:5])
+        for x, y in zip(*states):
+            assert np.array_equal(x, y)
+        assert np.array_equal(hist, np.array(each))
+        fit = ctx.fit()
+        for t in (1, 2, 3):
+            grid = {w: ctx.response(t, w).reshape(N, N) for w in range(10)}
+            tg = sampling.get_targets(ctx, t)
+            thr = p.MinParticlesPerBinForDispersionMeasurement * p.MType[t] / p.NType[t]
+            count = 3 if p.TypeOfVelocityStructure[t] in (0, 1) else 4
+            for k in range(count):  # r, t, p, q
+                v = misfit(grid[6 + k], tg[2 + k], grid[5], tg[1], level, thr, p.LowerDispLimit)
+                assert abs(fit[t][1 + k] - v * fit[t][5]) <= 1e-12 * abs(v * fit[t][5]), (t, k)
