@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "context.cuh"
+#include "stepmath.cuh"
 #include "galic_gpu.h"
 
 namespace {
@@ -54,7 +55,7 @@ namespace {
 constexpr int kSections = 8;       // FG_SECTIONS (allvars.h:123)
 constexpr int kBits = 21;          // BITS_PER_DIMENSION (allvars.h:213)
 constexpr int kMaxTreeLevel = 30;  // MAX_TREE_LEVEL (forcetree.h:16)
-constexpr int kWalkBlock = 256;
+constexpr int kWalkBlock = 64;     // (256: 12.9 against 12.5 ms a fill, means of two runs)
 
 // Peano-Hilbert state machine of peano.c:226-330: next state (kRot) and key
 // digit (kSub) for each state 0..47 and octant pix = 4*x + 2*y + z.  The
@@ -158,6 +159,24 @@ __global__ void k_keys(int n, const double *__restrict__ pos, double cx, double 
 
 // force_treeevaluate (forcetree_walk.c:12-222), mode 0, one probe per lane.
 // probes: SoA [3][np] in key order; res: SoA [4][np] (acc x, y, z, pot) * G.
+// 2^-200 <= |x| < 2^200: the operands of the walk's step_sqrt and step_div
+__device__ __forceinline__ bool walk_plain(double x)
+{
+  return ((unsigned) __double2hiint(x) & 0x7fffffffu) - 0x33700000u < 0x19000000u;
+}
+__device__ __noinline__ void walk_divide(double mass, double r2, double r, double *fac, double *wp)
+{
+  *fac = mass / (r2 * r);
+  *wp = -mass / r;
+}
+
+// What bounds the walk is FP64 issue and the chains of its square root and two
+// divisions; their general forms end basic blocks with tests of the operands.
+// The step's branch-free ones (same bits in walk_plain's range, the general
+// division out of line otherwise) took the walk of a fill of 1.2e6 masses
+// at 256 x 256 cells from 8.45 to 7.9 ms, the fill from 14.0 to 13.3.  Loading
+// both items that can follow while one is evaluated cost more registers than it
+// hid latency: 14.2 ms a fill.
 __global__ void __launch_bounds__(kWalkBlock) k_walk(const FillItem *__restrict__ items, int nitems, int np,
                                                     const double *__restrict__ probes, double hmax,
                                                     double theta, double G, double *__restrict__ res,
@@ -200,11 +219,14 @@ __global__ void __launch_bounds__(kWalkBlock) k_walk(const FillItem *__restrict_
     const double mass = it.mass;
     if(mass != 0.0) {
       n_int++;
-      const double r = sqrt(r2);
+      const bool plain = walk_plain(r2) && walk_plain(mass);
+      const double r = plain ? step_sqrt(r2) : sqrt(r2);
       double fac, wp;
       if(r >= hmax) {
-        fac = mass / (r2 * r);
-        wp = -mass / r;
+        unsigned ones = 0;
+        fac = step_div(mass, r2 * r, ones);
+        wp = step_div(-mass, r, ones);
+        if(!plain || step_ones(ones)) walk_divide(mass, r2, r, &fac, &wp);
       } else {
         const double u = r * h_inv;
         if(u < 0.5) {

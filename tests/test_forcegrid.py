@@ -164,6 +164,21 @@ def test_gpu_fill_matches_oracle(nh, nd, fg, theta, soft, seed):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("low,high", [(1e-80, 1e-80), (1e70, 1e70), (1e-70, 1e-50)])
+def test_gpu_fill_masses_outside_the_plain_range(low, high):
+    # the walk's branch-free division holds for masses of 2^-200 to 2^200; others
+    # (all of them, then some) take the general one
+    pos, mass = seeded_particles(3000, 1000, 4)
+    mass = mass * np.exp(np.linspace(np.log(low), np.log(high), len(mass)))
+    fp = forcegrid.fill_params(24, 0.05, 1.15, 43007.1, 0.2, 0.5, 4.0, 4)
+    st, *want = oracle_lib.oracle_force_grid_fill(fp, pos, mass)
+    assert st == 0
+    got = forcegrid.force_grid_fill(fp, pos, mass)
+    for g, w in zip(got[:3], want):
+        assert np.array_equal(g, w)
+
+
+@pytest.mark.gpu
 def test_gpu_fill_deterministic_and_coincident_rejected():
     fp, pos, mass, _ = load_fixture(FIXTURES[-1])
     a = forcegrid.force_grid_fill(fp, pos, mass)
