@@ -223,6 +223,12 @@ def sampling_inputs(model):
     return sp, tables
 
 
+def reference_built():
+    sys.path.insert(0, os.path.join(ROOT, "tests"))
+    import oracle_lib
+    return oracle_lib.reference_available()
+
+
 def _ref_sampling_timed(params, sp, ntarget, kind, tables):
     """GALIC's own sampling function (one rank) on the host; its progress
     output goes to /dev/null so that the bench's stdout stays one JSON line."""
@@ -992,14 +998,15 @@ def ours_arm(args, rank, world, local_rank):
     if rank == 0:
         peak = measured_fp64_peak(torch) if form == GALIC_FORM_FP64 else measured_fp32_peak(torch)
         kern_avg = sum(kern_ms) / len(kern_ms)
+        # the rows that time GALIC's own C beside theirs need it built
+        cpu_rows = world == 1 and args.cpu_seconds > 0 and reference_built()
         fill = measure_fill(model, args.steps, world == 1 and args.cpu_seconds > 0,
                             peak if form == GALIC_FORM_FP64 else measured_fp64_peak(torch))
-        target_sampling = measure_sampling(model, ctx, args.steps, world == 1 and args.cpu_seconds > 0)
-        jeans_solve = measure_jeans(model, args.steps, world == 1 and args.cpu_seconds > 0)
-        init_particles = measure_particles(model, args.steps, world == 1 and args.cpu_seconds > 0)
+        target_sampling = measure_sampling(model, ctx, args.steps, cpu_rows)
+        jeans_solve = measure_jeans(model, args.steps, cpu_rows)
+        init_particles = measure_particles(model, args.steps, cpu_rows)
         ensemble = measure_ensemble(args.ensemble_models, args.steps) if args.ensemble_models > 0 else None
-        construction = (measure_construction(args.construction, args.construction_scale,
-                                             world == 1 and args.cpu_seconds > 0)
+        construction = (measure_construction(args.construction, args.construction_scale, cpu_rows)
                         if args.construction != "none" else None)
         serving = (measure_serving(args.serve_requests, args.serve_gap, args.serve_scale, torch, args.serve_workers,
                                    args.serve_hbm_fraction)
@@ -1114,7 +1121,8 @@ def row_alone(args):
         res = measure_serving(args.serve_requests, args.serve_gap, args.serve_scale, torch, args.serve_workers,
                               args.serve_hbm_fraction)
     elif args.row == "construction":
-        res = measure_construction(args.construction, args.construction_scale, args.cpu_seconds > 0,
+        res = measure_construction(args.construction, args.construction_scale,
+                                   args.cpu_seconds > 0 and reference_built(),
                                    args.construction_window_gib)
     elif args.row == "fill":
         res = measure_fill(model, args.steps, False, measured_fp64_peak(torch))
