@@ -14,7 +14,7 @@
 //
 // The graph holds: accumulator and counter resets, the orbit kernel, and per
 // member the instantaneous-energy kernel, the fixed-point read-out and the
-// three merit kernels.  It captures the members' device pointers; any upload
+// fit.  It captures the members' device pointers; any upload
 // to a member (which may reallocate) invalidates the ensemble
 // (GALIC_ERR_STATE), and the caller builds a new one.
 #include <cuda_runtime.h>
