@@ -410,7 +410,7 @@ __device__ __forceinline__ void orbit_begin(const DevModel &M, const LogConsts &
   if(with_proj) proj = project(M, s.tovs, type, fc, s.x, s.v, sqrt(s.x[0] * s.x[0] + s.x[1] * s.x[1]));
   set_step(s, get_timestep(M, s.v, s.a, cell.iz * M.DG_Nbin + cell.iR));
   sink.enter(cell.iR, cell.iz);
-  sink.add(cell, 0.5 * s.dt, 0.0, proj);
+  sink.add(cell, 0.5 * s.dt, proj);
 }
 
 // What one position gives: the acceleration, the density-grid cell, the
@@ -605,9 +605,15 @@ __device__ __forceinline__ bool orbit_step(const DevModel &M, const LogConsts &L
     s.status = ORBIT_NONFINITE;
     more = false;
   }
-  if(more) set_step(s, T.dt);
-  sink.add(P.cell, 0.5 * dt, more ? 0.5 * s.dt : 0.0, T.proj);
-  return more;
+  if(!more) {
+    // the last half step alone: a second one of weight zero would turn the
+    // infinite projection of a position next to the axis into NaN
+    sink.add(P.cell, 0.5 * dt, T.proj);
+    return false;
+  }
+  set_step(s, T.dt);
+  sink.add(P.cell, 0.5 * dt, 0.5 * s.dt, T.proj);
+  return true;
 }
 
 // orbit_response.c:460-462: relative energy error of the finished orbit

@@ -105,10 +105,10 @@ struct ParkSink {
   }
   __device__ __forceinline__ void add(const Cell &k, double hdt, double next_hdt, const Proj &p)
   {
-    add_one(k, hdt, p);
-    add_one(k, next_hdt, p);
+    add(k, hdt, p);
+    add(k, next_hdt, p);
   }
-  __device__ __forceinline__ void add_one(const Cell &k, double hdt, const Proj &p)
+  __device__ __forceinline__ void add(const Cell &k, double hdt, const Proj &p)
   {
     const double w[4] = {hdt * (1 - k.fR) * (1 - k.fz), hdt * (k.fR) * (1 - k.fz), hdt * (1 - k.fR) * (k.fz),
                          hdt * (k.fR) * (k.fz)};

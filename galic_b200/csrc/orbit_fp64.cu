@@ -99,6 +99,21 @@ struct DenseSink {
       }
     }
   }
+  __device__ __forceinline__ void add(const Cell &cell, double hdt, const Proj &p)
+  {
+    double w[4];
+    slot_weights(cell, hdt, w);
+#pragma unroll
+    for(int k = 0; k < 4; k++) {
+      c[k][0] = c[k][0] + w[k];
+      if(with_egy) {
+        c[k][1] = c[k][1] + w[k] * p.vr2;
+        c[k][2] = c[k][2] + w[k] * p.vt2;
+        c[k][3] = c[k][3] + w[k] * p.vq2;
+        c[k][4] = c[k][4] + w[k] * p.vp2;
+      }
+    }
+  }
   __device__ __forceinline__ void finish()
   {
     const bool all[4] = {true, true, true, true};
@@ -216,6 +231,19 @@ struct NodeSink64 {
       a[k][2] = fma(n[k], p.vt2, fma(w[k], p.vt2, a[k][2]));
       a[k][3] = fma(n[k], p.vq2, fma(w[k], p.vq2, a[k][3]));
       a[k][4] = fma(n[k], p.vp2, fma(w[k], p.vp2, a[k][4]));
+    }
+  }
+  __device__ __forceinline__ void add(const Cell &cell, double hdt, const Proj &p)
+  {
+    double w[4];
+    slot_weights(cell, hdt, w);
+#pragma unroll
+    for(int k = 0; k < 4; k++) {
+      a[k][0] = a[k][0] + w[k];
+      a[k][1] = fma(w[k], p.vr2, a[k][1]);
+      a[k][2] = fma(w[k], p.vt2, a[k][2]);
+      a[k][3] = fma(w[k], p.vq2, a[k][3]);
+      a[k][4] = fma(w[k], p.vp2, a[k][4]);
     }
   }
 };

@@ -153,3 +153,22 @@ def test_orbits_outside_the_step_ranges_equal_the_oracle(shape):
                 assert got[0] == want[0] and got[1] == want[1]
                 for a, b in zip(got[2:], want[2:7]):
                     assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.gpu
+def test_infinite_projections_stay_infinite():
+    """A start so close to the axis that R underflows to 0: the tangential projections are infinite, and so are the
+    oracle's bins of the first half step; every bin, the time and the orbit count."""
+    m = synth.config_halo_disk(24, 8, level=5, seed=3)
+    o = Oracle(m.params, use_libm=False)
+    o.load_model(m)
+    start = np.array([1e-200, 2e-200, m.pos[0][2]])
+    with Context(m.params) as ctx:
+        ctx.load_model(m)
+        for t in (1, 2):
+            got = ctx.produce_orbit_response_field_mod(start, m.vel[0], m.mass[0], m.tint[0], t)
+            want = o.orbit_mod(start, np.ascontiguousarray(m.vel[0]), m.mass[0], m.tint[0], t)
+            assert any(np.isinf(b).any() for b in want[2:7])
+            assert got[0] == want[0] and got[1] == want[1]
+            for a, b in zip(got[2:], want[2:7]):
+                assert np.array_equal(a, b, equal_nan=True)
