@@ -78,7 +78,13 @@ __device__ __forceinline__ Cell32 cell32(float br, float bz, int nbin, float bma
 }
 
 // acceleration (grid.c:122-197) and streaming velocity (disp_fields.c:118-132)
-// at x; both read the same float4 table corners
+// at x; both read the same float4 table corners.  The roundings of the
+// streaming velocity's sum are spelled out, because the projections subtract
+// it from a velocity of nearly its size: left to the compiler, the product
+// that is rounded on its own changed with the code around an orbit's start
+// (3e-11 of a grid's peak).  The pass rounds another one at the starts
+// (PASS_START) than everywhere else.
+template <bool PASS_START>
 __device__ __forceinline__ void accel32(const Model32 &M, int type, const float *x, float *a, float *vstr)
 {
   const float R2 = x[0] * x[0] + x[1] * x[1];
@@ -95,7 +101,8 @@ __device__ __forceinline__ void accel32(const Model32 &M, int type, const float 
   const float4 qV = M.vstream_zero[type] ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldg(&Q[2]);
   const float w00 = (1.f - c.fR) * (1.f - c.fz), w01 = c.fR * (1.f - c.fz);
   const float w10 = (1.f - c.fR) * c.fz, w11 = c.fR * c.fz;
-  *vstr = qV.x * w00 + qV.z * w10 + qV.y * w01 + qV.w * w11;
+  const float v0 = PASS_START ? fmaf(qV.z, w10, __fmul_rn(qV.x, w00)) : fmaf(qV.x, w00, __fmul_rn(qV.z, w10));
+  *vstr = fmaf(qV.w, w11, fmaf(qV.y, w01, v0));
   a[0] = a[1] = a[2] = 0.f;
   if(M.tabulated) {
     if(jd < M.fgmax && id < M.fgmax) {
@@ -145,9 +152,10 @@ __device__ __forceinline__ Proj32 project32(int tovs, const float *x, const floa
     const float vdx = v[0] * x[0] + v[1] * x[1];
     const float ir2 = frcp(r2);
     o.vr2 = vdx * vdx * ir2;
-    const float vq = (v[1] * x[0] - v[0] * x[1]) * rsqrtf(r2);
+    const float vq = __fmul_rn(v[1] * x[0] - v[0] * x[1], rsqrtf(r2));
+    const float vp = __fsub_rn(vq, vstr);
     o.vq2 = vq * vq;
-    o.vp2 = (vq - vstr) * (vq - vstr);
+    o.vp2 = vp * vp;
     o.vt2 = v[2] * v[2];
   } else {
     // Q = x cross (0,0,-1) = (-y, x, 0); T = x cross Q
@@ -155,9 +163,10 @@ __device__ __forceinline__ Proj32 project32(int tovs, const float *x, const floa
     const float vdx = v[0] * x[0] + v[1] * x[1] + v[2] * x[2];
     o.vr2 = vdx * vdx * frcp(r2);
     const float q2 = x[0] * x[0] + x[1] * x[1];
-    const float vq = (v[1] * x[0] - v[0] * x[1]) * rsqrtf(q2);
+    const float vq = __fmul_rn(v[1] * x[0] - v[0] * x[1], rsqrtf(q2));
+    const float vp = __fsub_rn(vq, vstr);
     o.vq2 = vq * vq;
-    o.vp2 = (vq - vstr) * (vq - vstr);
+    o.vp2 = vp * vp;
     const float T0 = x[0] * x[2], T1 = x[1] * x[2], T2 = -q2;
     const float t2 = T0 * T0 + T1 * T1 + T2 * T2;
     const float vdT = v[0] * T0 + v[1] * T1 + v[2] * T2;
@@ -294,7 +303,9 @@ struct State32 {
 
 enum { LANE_ACTIVE = 0, LANE_FINISH = 1, LANE_DONE = 2, LANE_LAST = 3, LANE_START = 4 };
 
-// orbit_response.c:172-206 in FP32: initial state of one orbit
+// orbit_response.c:172-206 in FP32: initial state of one orbit (PASS: of the
+// batched pass)
+template <bool PASS>
 __device__ __forceinline__ void orbit32_init(const Model32 &M, State32 &s, const double *xd, const double *vd,
                                              int type, double timespan)
 {
@@ -314,7 +325,7 @@ __device__ __forceinline__ void orbit32_init(const Model32 &M, State32 &s, const
   s.steps = 0;
   s.status = ORBIT_OK;
   float vstr;
-  accel32(M, type, s.x, s.a, &vstr);
+  accel32<PASS>(M, type, s.x, s.a, &vstr);
   Cell32 c = density_cell32(M, s.x);
   s.iR = c.iR;
   s.iz = c.iz;
@@ -353,7 +364,7 @@ __device__ __forceinline__ bool orbit32_step(const Model32 &M, State32 &s, Sink 
 #pragma unroll
   for(int i = 0; i < 3; i++) comp_add(s.x[i], s.xc[i], fdt * (s.v[i] - s.vc[i]));
   float vstr;
-  accel32(M, s.type, s.x, s.a, &vstr);
+  accel32<false>(M, s.type, s.x, s.a, &vstr);
 #pragma unroll
   for(int i = 0; i < 3; i++) comp_add(s.v[i], s.vc[i], hdt * s.a[i]);
   Cell32 c = density_cell32(M, s.x);
@@ -552,7 +563,7 @@ __device__ __forceinline__ void calc_all_fp32_body(const Src &S)
       xd[i] = P.pos[3 * p + i];
       vd[i] = P.vel[3 * p + i];
     }
-    orbit32_init(M, s, xd, vd, type, P.tint[p]);
+    orbit32_init<true>(M, s, xd, vd, type, P.tint[p]);
     const DevModel &M64 = S.model64(mi);
     aux.E0 = 0.5 * (vd[0] * vd[0] + vd[1] * vd[1] + vd[2] * vd[2]) + forcegrid_pot(M64, pot_logs(M64), xd);
     return true;
@@ -660,7 +671,7 @@ __global__ void __launch_bounds__(128) k_orbits_dense_fp32(const __grid_constant
   sink.Nb = M.DG_Nbin;
   State32 s;
   const double *xd = &b.pos[3 * k], *vd = &b.vel[3 * k];
-  orbit32_init(M, s, xd, vd, b.type[k], b.timespan[k]);
+  orbit32_init<false>(M, s, xd, vd, b.type[k], b.timespan[k]);
   const LogConsts L = pot_logs(M64);
   double x0[3] = {xd[0], xd[1], xd[2]};
   const double E0 = 0.5 * (vd[0] * vd[0] + vd[1] * vd[1] + vd[2] * vd[2]) + forcegrid_pot(M64, L, x0);
