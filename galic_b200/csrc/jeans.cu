@@ -208,12 +208,15 @@ __global__ void __launch_bounds__(256) k_sph_march(const __grid_constant__ Jeans
         bool heun = true, plain = true;
         for(int t = threadIdx.x; t < SPH_STEPS; t += 32) {
           heun = heun && c[t].flag == 2;
-          plain = plain && c[t].c0 == 0 && c[t].c1 == 0;
+          plain = plain && c[t].c0 == 0 && c[t].c1 == 0 && gm_fabs(c[t].a0) < 0x1p+500 &&
+                  gm_fabs(c[t].a1) < 0x1p+500 && gm_fabs(c[t].dr) < 0x1p+400;
         }
         heun = __all_sync(0xffffffffu, heun);
         plain = __all_sync(0xffffffffu, plain);
         if(threadIdx.x) continue;
-        if(heun && plain && gm_fabs(y) < GM_INF) {
+        // (within these bounds y and ypred stay finite throughout the interval:
+        // a zero times infinity would be NaN)
+        if(heun && plain && gm_fabs(y) < 0x1p+1000) {
 #pragma unroll 10
           for(int t = 0; t < SPH_STEPS; t++) y += c[t].dr * 0.5 * (c[t].a0 + c[t].a1);
         } else if(heun) {

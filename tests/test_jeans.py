@@ -149,3 +149,19 @@ def test_gpu_tilted_march_column_counts(fg_nbin):
     assert st == 0
     for w, name in enumerate(_ffi.JEANS_TABLES):
         assert np.array_equal(got[2][name], ref[2, w], equal_nan=True), name
+
+
+@pytest.mark.gpu
+def test_gpu_infinite_force_gives_the_restatements_tables():
+    """An infinite entry of the force table at z = 0: the spherical march meets infinite coefficients, after which
+    the reference's products of them with a zero anisotropy are NaN."""
+    m = jeans_model(tovs=(0, 3, 0))
+    m.dpotdr[20] = -np.inf
+    sp, jp = jeans_params(m, 0.0, 0.0)
+    got, _ = _gpu_dispfield(m, sp, jp)
+    with np.errstate(all="ignore"):
+        st, ref = oracle_lib.oracle_dispfield(m, sp, jp, use_libm=False)
+    assert st == 0 and np.isnan(ref[1, 0]).any()
+    for t in (1, 2, 3):
+        for w, name in enumerate(_ffi.JEANS_TABLES):
+            assert np.array_equal(got[t][name], ref[t, w], equal_nan=True), (t, name)
