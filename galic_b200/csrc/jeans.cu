@@ -777,6 +777,10 @@ extern "C" int galic_calculate_dispfield(galic_ctx *ctx, const galic_sample_para
   const int pitch = N <= 384 / 32 * TILT_OWN ? 384 / 32 * TILT_OWN : (N <= 768 / 32 * TILT_OWN ? 768 / 32 * TILT_OWN : 1024);
   const size_t row_doubles = (size_t) TILT_STEPS * TC_ROWS * pitch;
   const int tilt_rows = (int) std::max<size_t>(1, std::min<size_t>(N - 1, (32ull << 20) / (row_doubles * sizeof(double))));
+  // types whose integrand points are held at once: all of them within 256 MiB
+  // (27 MB a type at N = 256, 428 MB at N = 1024)
+  const size_t axi_bytes = (size_t) N * (N + 1) * (AXI_STEPS + 1) * sizeof(double);
+  const int axi_types = (int) std::max<size_t>(1, std::min<size_t>(3, (256ull << 20) / axi_bytes));
   std::vector<double> Rg(2 * N + 3);
   for(int j = 0; j < 2 * N + 3; j++) Rg[j] = p.FG_Rmin * (std::pow(p.FG_Fac, j) - 1.0);
   bool any_tilt = false;
@@ -813,8 +817,8 @@ extern "C" int galic_calculate_dispfield(galic_ctx *ctx, const galic_sample_para
   }
   if(nt == 0) goto done;
   JCK(cudaMallocAsync((void **) &d_sph, (size_t) nt * (N + 1) * SPH_STEPS * sizeof(SphCoef), s));
-  JCK(cudaMallocAsync((void **) &d_Y, (size_t) nt * N * (N + 1) * (AXI_STEPS + 1) * sizeof(double), s));
-  JCK(cudaMallocAsync((void **) &d_S, (size_t) nt * N * (N + 1) * sizeof(double), s));
+  JCK(cudaMallocAsync((void **) &d_Y, axi_types * axi_bytes, s));
+  JCK(cudaMallocAsync((void **) &d_S, (size_t) axi_types * N * (N + 1) * sizeof(double), s));
   if(any_tilt) {
     JCK(cudaMallocAsync((void **) &d_q, G * sizeof(double), s));
     JCK(cudaMallocAsync((void **) &d_tilt, 2 * tilt_rows * row_doubles * sizeof(double), s));
@@ -829,15 +833,20 @@ extern "C" int galic_calculate_dispfield(galic_ctx *ctx, const galic_sample_para
     // ev2[2]: everything the second stream reads is in place
     JCK(cudaEventRecord(ctx->ev2[2], s));
     JCK(cudaStreamWaitEvent(s2, ctx->ev2[2], 0));
-    // spherical and axisymmetric parts (disp_fields.c:512-729), all types at
-    // once; queued behind the first block of tilted coefficients
+    // spherical and axisymmetric parts (disp_fields.c:512-729), axi_types
+    // types at once; queued behind the first block of tilted coefficients
     auto first_parts = [&]() {
-      k_axi_points<<<dim3(blocks((long long) N * (N + 1) * (AXI_STEPS + 1), 256), nt), 256, 0, s2>>>(T, d_jd, d_Y);
-      k_axi_sums<<<dim3(blocks((long long) N * (N + 1), 128), nt), 128, 0, s2>>>(T, d_Y, d_S);
-      k_axi_march<<<dim3(blocks(N, 32), nt), 32, 0, s2>>>(T, d_S);
-      k_axi_divide<<<dim3(blocks((long long) G, 256), nt), 256, 0, s2>>>(T);
-      k_axi_stream<<<dim3(blocks((long long) G, 256), nt), 256, 0, s2>>>(T);
-      launches += 5;
+      for(int i0 = 0; i0 < nt; i0 += axi_types) {
+        const int k = std::min(axi_types, nt - i0);
+        JeansTypes P{};
+        std::copy(T.t + i0, T.t + i0 + k, P.t);
+        k_axi_points<<<dim3(blocks((long long) N * (N + 1) * (AXI_STEPS + 1), 256), k), 256, 0, s2>>>(P, d_jd, d_Y);
+        k_axi_sums<<<dim3(blocks((long long) N * (N + 1), 128), k), 128, 0, s2>>>(P, d_Y, d_S);
+        k_axi_march<<<dim3(blocks(N, 32), k), 32, 0, s2>>>(P, d_S);
+        k_axi_divide<<<dim3(blocks((long long) G, 256), k), 256, 0, s2>>>(P);
+        k_axi_stream<<<dim3(blocks((long long) G, 256), k), 256, 0, s2>>>(P);
+        launches += 5;
+      }
     };
     k_sph_coef<<<dim3(blocks((long long) (N + 1) * SPH_STEPS, 256), nt), 256, 0, any_tilt ? s2 : s>>>(T, d_sph);
     if(!any_tilt) {

@@ -165,3 +165,22 @@ def test_gpu_infinite_force_gives_the_restatements_tables():
     for t in (1, 2, 3):
         for w, name in enumerate(_ffi.JEANS_TABLES):
             assert np.array_equal(got[t][name], ref[t, w], equal_nan=True), (t, name)
+
+
+@pytest.mark.gpu
+def test_gpu_large_grids_hold_the_points_of_few_types():
+    """529^2 with three types: their integrand points (114 MB each) take turns in 256 MiB; all tables as the
+    restatement's, and the call's memory as it was when types ran one by one (tables, coefficients, 256 MiB)."""
+    from pool_lib import PoolMark
+    N = 529
+    m = jeans_model(fg_nbin=N, tovs=(1, 2, 3))
+    sp, jp = jeans_params(m)
+    mark = PoolMark()
+    got, _ = _gpu_dispfield(m, sp, jp)
+    # the call's 4 x 8 tables, the context's 15 of them and its force, streaming and potential tables
+    assert mark.bytes() <= 8 * N * N * (32 + 15 + 8) + (256 + 64 + 32 << 20)
+    st, ref = oracle_lib.oracle_dispfield(m, sp, jp, use_libm=False)
+    assert st == 0
+    for t in (1, 2, 3):
+        for w, name in enumerate(_ffi.JEANS_TABLES):
+            assert np.array_equal(got[t][name], ref[t, w], equal_nan=True), (t, name)
