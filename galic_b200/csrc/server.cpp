@@ -29,6 +29,7 @@
 #include <thread>
 #include <vector>
 
+#include "footprint.h"
 #include "galic_gpu.h"
 
 namespace galic_internal {
@@ -64,13 +65,17 @@ size_t job_count(const galic_job_t &d)
   return std::min((size_t) d.n, (size_t) (1 + d.fraction_per_rep * d.n));
 }
 
-// device bytes of the per-orbit grids of one window of repetitions: the
-// whole iteration, capped at 8 GiB (at least one repetition); a job holds
-// two windows at once (galic_optimize_reps)
+// a repetition's share of galic_optimize_reps' window_bytes
+size_t job_rep_bytes(const galic_job_t &d)
+{
+  return job_count(d) * 2 * (5 * galic_footprint::bins(d.prm->DG_MaxLevel) * 8 + 128);
+}
+
+// window_bytes of a job: the whole iteration, capped at 8 GiB (at least one
+// repetition); a job holds two windows at once (galic_optimize_reps)
 size_t job_window_bytes(const galic_job_t &d)
 {
-  const size_t G = (size_t) 1 << (2 * d.prm->DG_MaxLevel);
-  const size_t per_rep = job_count(d) * 2 * (5 * G * 8 + 128);
+  const size_t per_rep = job_rep_bytes(d);
   const size_t iter = per_rep * (size_t) std::max(d.reps_per_iteration, 1);
   return std::max(per_rep, std::min(iter, (size_t) 8 << 30));
 }
@@ -209,15 +214,13 @@ extern "C" size_t galic_job_device_bytes(const galic_job_t *job)
 {
   if(!job || !job->prm || job->n <= 0) return 0;
   const galic_params_t &p = *job->prm;
-  const size_t n = (size_t) job->n;
-  const size_t NF = (size_t) p.FG_Nbin * p.FG_Nbin;
-  const size_t G = (size_t) 1 << (2 * p.DG_MaxLevel);
-  const size_t Ns = (((size_t) 1 << (2 + 2 * p.DG_MaxLevel)) - 1) / 3;
-  size_t b = n * 160;                       // particle state (allvars.h:844-868) and processing order
-  b += NF * (16 + 8 + 3 * 8 + 3 * 64);      // FP64 force tables, streaming velocities, FP32 quad tables
-  b += G * (8 + 4 + 320 + 640) + Ns * 520;  // geometry, committed grids, fixed point, stacks, targets
-  b += 2 * job_window_bytes(*job) + job_count(*job) * 64;  // per-orbit grids of two windows of repetitions
-  b += (size_t) 16 << 20;                   // fit scratch, allocator granularity
+  const size_t reps = (size_t) std::max(job->reps_per_iteration, 1);
+  const size_t count = job_count(*job);
+  // particles of one window: all distinct
+  const size_t window = std::min(job_window_bytes(*job) / job_rep_bytes(*job), (size_t) job->n / count) * count;
+  size_t b = galic_footprint::context(p.FG_Nbin, p.DG_MaxLevel);
+  b += galic_footprint::particles((size_t) job->n, 2 * galic_footprint::window(window, p.DG_MaxLevel) + reps * count * 4);
+  b += (size_t) 16 << 20;  // counters, sort histograms, allocator granularity
   return b;
 }
 

@@ -86,3 +86,42 @@ def test_oversize_job_rejected_and_early_stop():
         r = s.wait(s.submit(models[1], form=GALIC_FORM_FP64, max_iterations=5, reps_per_iteration=2,
                             fraction_per_rep=0.003, converge_rel=1.0))
         assert r["status"] == 0 and r["iterations"] == 1 and r["reps"] == 2
+
+
+def job_bytes(model, n, fraction, reps):
+    job = _ffi.GalicJob()
+    job.prm = C.pointer(model.params)
+    job.n, job.fraction_per_rep, job.reps_per_iteration = n, fraction, reps
+    return int(_ffi.load_library().galic_job_device_bytes(C.byref(job)))
+
+
+def test_job_bytes_hold_two_full_windows():
+    """A schedule whose iteration exceeds the 8 GiB of a window: two windows, every array of their particles and the
+    context's own fit the reservation."""
+    level, n, fraction, reps = 1, 20_000_000, 0.01, 100
+    m = synth.config_halo(n=32, level=level, seed=1)
+    count, G = 1 + int(fraction * n), 4 ** level
+    window = (8 << 30) // (count * 2 * (40 * G + 128)) * count
+    assert window < reps * count
+    orbit = 40 * G + 24 + 24 + 8 + 8 + 8 + 8 + 4 + 4 + 4 + 8  # grids, pos, vel, mass, time, tall, error, type, orbits, status, steps
+    trial = 4 + 3 * 4 + 3 * 4 + 4 * 8 + 3 * 8 + 18 * 8 + 2 * 8 + 4 * 8 + 24  # index, lists, lengths, try_disp, vel_try, F, fac, inst_v, cell
+    particle = 24 + 24 + 8 + 8 + 8 + 32 + 32 + 4 + 4 + 4
+    assert job_bytes(m, n, fraction, reps) >= 2 * window * (2 * orbit + trial) + n * particle + reps * count * 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [GALIC_FORM_FP64, GALIC_FORM_FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("level,n,fraction,reps", [(7, 3000, 0.05, 1), (7, 3000, 0.05, 6), (5, 200000, 0.0, 1),
+                                                   (4, 60000, 0.6, 3), (3, 20000, 0.2, 4)])
+def test_jobs_stay_within_their_reservation(level, n, fraction, reps, form):
+    """The most a job takes from the allocator, against what its admission counts."""
+    from pool_lib import PoolMark
+    m = synth.config_halo(n=n, level=level, seed=31)
+    want = job_bytes(m, n, fraction, reps)
+    mark = PoolMark()
+    with Server(64 << 30, workers=1) as s:
+        r = s.wait(s.submit(m, form=form, max_iterations=2, reps_per_iteration=reps, fraction_per_rep=fraction, seed=3))
+    assert r["status"] == 0
+    assert mark.bytes() <= want
+    # not far above it either: at most two windows of the whole iteration instead of one, and the allowance
+    assert want <= 2 * mark.bytes() + (40 << 20)
