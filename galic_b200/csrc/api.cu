@@ -17,6 +17,7 @@
 #include "galic_gpu.h"
 #include "kernels.cuh"
 #include "rep.cuh"
+#include "windows.h"
 
 
 namespace {
@@ -1201,12 +1202,7 @@ extern "C" int galic_optimize_reps(galic_ctx *ctx, const int *idx, int count, in
     ctx->idx_cap = (size_t) reps * count;
   }
   CK(second_stream(ctx));
-  // a window's orbit launch lasts as long as its longest orbit: while two
-  // windows' orbits leave the GPU room, they run at once, on a stream each
-  // (the FP32 composite construction of 6432 orbits in
-  // two windows: 53 -> 45.5 ms).  Larger
-  // ones would only share it (20 000 orbits a window: 0.69 s against 0.66 s).
-  const bool pair = 2 * maxM <= 8192;
+  const bool pair = windows_paired(wins.size(), maxM);
   if(pair && !ctx->stream3)
     CK(cudaStreamCreateWithPriority(&ctx->stream3, cudaStreamNonBlocking, ctx->priority));
   // every index of the call in one copy; staged through pinned memory
