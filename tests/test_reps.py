@@ -182,3 +182,78 @@ def test_fit_at_every_depth_of_the_pyramid(level):
             for k in range(count):  # r, t, p, q
                 v = misfit(grid[6 + k], tg[2 + k], grid[5], tg[1], level, thr, p.LowerDispLimit)
                 assert abs(fit[t][1 + k] - v * fit[t][5]) <= 1e-12 * abs(v * fit[t][5]), (t, k)
+
+
+def short_orbits(n_halo, n_disk, level, seed):
+    """A halo + disk whose orbits take a few dozen steps."""
+    m = synth.config_halo_disk(n_halo=n_halo, n_disk=n_disk, level=level, seed=seed)
+    m.tint = m.tint * 0.05
+    return m
+
+
+@pytest.mark.parametrize("form", [GALIC_FORM_FP64, GALIC_FORM_FP32], ids=["fp64", "fp32"])
+def test_large_windows_equal_sequential_repetitions(form):
+    """Three windows of 4500 particles each, more than run two at a time, the second with particles of the first."""
+    m = short_orbits(6000, 1000, 4, 58)
+    lists = cycling_lists(m.n, 1500, 9, 6)  # slots 7000 on repeat those from slot 0
+    results = []
+    for windows in (False, True):
+        with Context(m.params) as ctx:
+            ctx.load_model(m)
+            ctx.calc_all_response_fields(form)
+            if windows:
+                ctx.optimize_reps(lists, 5, 30, form, window_bytes=3 * 1500 * 2 * (5 * 256 * 8 + 128))
+            else:
+                for r in range(len(lists)):
+                    ctx.optimize_rep(lists[r], 5, 30 + r, form)
+            results.append(state(ctx, (1, 2)))
+    for x, y in zip(*results):
+        assert np.array_equal(np.asarray(x), np.asarray(y), equal_nan=True)
+    assert results[0][5][1].sum() > 0
+
+
+@pytest.mark.parametrize("count", [2467, 14501])
+def test_many_particles_in_one_repetition(count):
+    """More particles than the acceptance's CTA has threads, more acceptances of a type than the commit stages at
+    once and (14501) more orbits than the spread launch has lanes: the committed grids restated, addition by
+    addition in particle order, from the accepted particles' single orbits, and the repetition as a window."""
+    m = short_orbits(13001, 3000, 3, 59)
+    idx = np.random.default_rng(7).permutation(m.n)[:count].astype(np.int32)
+    with Context(m.params) as ctx:
+        ctx.load_model(m)
+        ctx.calc_all_response_fields(GALIC_FORM_FP64)
+        before = {t: [ctx.response(t, w) for w in range(10)] for t in (1, 2)}
+        vel0, orbits0, vdisp0 = ctx.particles()
+        ctx.optimize_rep(idx, 8, 3)
+        vel1, orbits1, vdisp1, _, _, (tries, changes) = first = state(ctx, (1, 2))
+        after = {t: [ctx.response(t, w) for w in range(10)] for t in (1, 2)}
+        took = np.any(vel0 != vel1, axis=1)
+        assert not took[np.setdiff1d(np.arange(m.n), idx)].any()
+        for t in (1, 2):
+            assert tries[t] == np.sum(m.ptype[idx] == t) and changes[t] == np.sum(took & (m.ptype == t))
+        assert changes[1] > 256 and (count < 10000 or changes[2] > 256)
+        for t in (1, 2):
+            delta = np.zeros((5, 64))
+            for k in idx[(m.ptype[idx] == t) & took[idx]]:
+                old = ctx.produce_orbit_response_field_mod(m.pos[k], vel0[k], m.mass[k], m.tint[k], t)
+                new = ctx.produce_orbit_response_field_mod(m.pos[k], vel1[k], m.mass[k], m.tint[k], t)
+                delta += np.stack(new[2:]) - np.stack(old[2:])
+                assert orbits1[k] == new[1]
+            for w in range(5):
+                assert np.array_equal(after[t][w], before[t][w] + delta[w]), (t, w)
+            assert np.array_equal(after[t][5], before[t][5])
+            # the energy grid: every change of the projections lands on the four nodes of a cell with weights that
+            # sum to one, so the grids' sums change by the particles' changes
+            sel = took & (m.ptype == t)
+            dv = (vdisp1[sel] - vdisp0[sel]) * m.mass[sel][:, None]
+            for a in range(4):  # r, t, p, q
+                got = np.sum(after[t][6 + a]) - np.sum(before[t][6 + a])
+                scale = np.sum(np.abs(dv[:, a])) + np.sum(np.abs(before[t][6 + a]))
+                # sums of at most 14501 terms of either sign, each rounded once
+                assert abs(got - np.sum(dv[:, a])) <= 14501 * 2.0 ** -53 * 4 * scale, (t, a)
+    with Context(m.params) as ctx:
+        ctx.load_model(m)
+        ctx.calc_all_response_fields(GALIC_FORM_FP64)
+        ctx.optimize_reps(idx[None], 8, 3)
+        for x, y in zip(first, state(ctx, (1, 2))):
+            assert np.array_equal(np.asarray(x), np.asarray(y), equal_nan=True)
