@@ -35,12 +35,12 @@ __device__ __forceinline__ StepFloor step_floor(double x)
 // a / b, correctly rounded: the reciprocal by two Newton steps from the
 // hardware's approximation (2^-20 relative or better), the quotient and one
 // fused correction with the exact remainder (Markstein, IBM J. Res. Develop.
-// 34(1), 1990).  2^-500 <= |b| <= 2^500, a = 0 or 2^-960 <= |a| and |a / b| <=
-// 2^960 (a zero quotient is +0).  Divisors whose significand is next to 2 are
-// the method's exception (their reciprocals lie next to rounding boundaries,
-// and Newton's steps approach them from below): `ones` collects the largest
-// top 20 fraction bits, and the quotient may be off by an ulp when
-// step_ones(ones).
+// 34(1), 1990).  2^-500 <= |b| <= 2^500; a = 0 (for b > 0 the quotient is +0,
+// whichever zero a is) or both |a| and |a / b| in [2^-960, 2^960].  Divisors
+// whose significand is next to 2 are the method's exception (their reciprocals
+// lie next to rounding boundaries, and Newton's steps approach them from
+// below): `ones` collects the largest top 20 fraction bits, and the quotient
+// may be off by an ulp when step_ones(ones).
 __device__ __forceinline__ double step_div(double a, double b, unsigned &ones)
 {
   ones = max(ones, __double2hiint(b) & 0xfffffu);

@@ -172,3 +172,89 @@ def test_infinite_projections_stay_infinite():
             assert got[0] == want[0] and got[1] == want[1]
             for a, b in zip(got[2:], want[2:7]):
                 assert np.array_equal(a, b, equal_nan=True)
+
+
+BITS_SRC = r'''
+#include "gmath.h"
+#include "stepmath.cuh"
+__device__ bool same(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
+__global__ void k_bits(int n, const double *a, const double *b, int what, unsigned *bad)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if(i >= n) return;
+  const double x = a[i], y = b[i];
+  bool ok = true;
+  unsigned ones = 0;  // operands the functions refuse
+  if(what == 0) {
+    const double q = step_div(x, y, ones);
+    ok = same(q, x == 0 && y > 0 ? 0.0 : x / y) || step_ones(ones);
+  }
+  if(what == 1) ok = same(step_sqrt(x), sqrt(x));
+  if(what == 2) ok = same(step_log(x), gm_log(x));
+  if(what == 3) {
+    double s, c, s0, c0;
+    step_direction(x, y, &s, &c, ones);
+    gm_sincos(gm_atan2(x, y), &s0, &c0);
+    ok = (same(s, s0) && same(c, c0)) || step_ones(ones);
+  }
+  if(!ok) atomicAdd(bad, 1u);
+}
+extern "C" int compare_bits(int n, const double *a, const double *b, int what)
+{
+  double *da, *db;
+  unsigned *bad, h = 0;
+  if(cudaMalloc(&da, n * 8) || cudaMalloc(&db, n * 8) || cudaMalloc(&bad, 4)) return -1;
+  cudaMemcpy(da, a, n * 8, cudaMemcpyHostToDevice);
+  cudaMemcpy(db, b, n * 8, cudaMemcpyHostToDevice);
+  cudaMemset(bad, 0, 4);
+  k_bits<<<(n + 255) / 256, 256>>>(n, da, db, what, bad);
+  if(cudaMemcpy(&h, bad, 4, cudaMemcpyDeviceToHost)) return -1;
+  cudaFree(da); cudaFree(db); cudaFree(bad);
+  return (int) h;
+}
+'''
+
+
+def _whole_range(what, rng, n):
+    """Operands over all of the header's stated ranges, their ends among them."""
+    sign = rng.choice([-1.0, 1.0], n)
+    pick = lambda lo, hi: np.where(rng.random(n) < 0.05, rng.choice([lo, hi], n), rng.integers(lo, hi + 1, n))
+    if what == 0:
+        eb = pick(-500, 500)
+        b = np.where(eb == 500, 2.0 ** 500, np.ldexp(_significands(rng, n), eb))
+        ea = pick(-960, 959)
+        ea = np.clip(ea, eb - 958, eb + 958)  # the quotient's exponent is ea - eb or one less
+        a = np.ldexp(_significands(rng, n), np.clip(ea, -960, 959))
+        # squares of cancelled sums, as the projections have them, over sums of squares
+        x, y, u, v = (np.ldexp(_significands(rng, n), rng.integers(-100, 100, n)) for _ in range(4))
+        d = x * y - (x * y) * (1 + rng.integers(-3, 4, n) * 2.0 ** -52)
+        kind = rng.random(n)
+        a = np.where(kind < 0.2, d * d, np.where(kind < 0.25, 0.0, a))
+        b = np.where(kind < 0.2, x * x + y * y, b)
+        return a * sign, np.where(rng.random(n) < 0.5, b, -b)
+    if what == 1:
+        return np.where(rng.random(n) < 0.02, rng.choice([2.0 ** -900, 2.0 ** 900], n),
+                        np.ldexp(_significands(rng, n), pick(-900, 899))), np.ones(n)
+    if what == 2:
+        return np.ldexp(_significands(rng, n), pick(0, 999)), np.ones(n)
+    return np.ldexp(_significands(rng, n), pick(-100, 99)) * sign, np.ldexp(_significands(rng, n), pick(-100, 99)) * \
+        rng.choice([-1.0, 1.0], n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", [0, 1, 2, 3], ids=["div", "sqrt", "log", "direction"])
+def test_step_functions_equal_the_general_ones_over_their_ranges(tmp_path_factory, what):
+    d = tmp_path_factory.mktemp("bits")
+    (d / "t.cu").write_text(BITS_SRC)
+    subprocess.run(["/usr/local/cuda/bin/nvcc", "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "--fmad=false", "-shared", "-Xcompiler", "-fPIC", "-I", os.path.join(ROOT, "galic_b200", "csrc"),
+                    str(d / "t.cu"), "-o", str(d / "libt.so")], check=True)
+    a, b = _whole_range(what, np.random.default_rng(40 + what), 4_000_000)
+    a, b = np.ascontiguousarray(a, dtype=np.float64), np.ascontiguousarray(b, dtype=np.float64)
+    if what == 0:  # nothing outside the stated range
+        nz = a != 0
+        q = np.abs(a[nz] / b[nz])
+        assert 2.0 ** -500 <= np.abs(b).min() and np.abs(b).max() <= 2.0 ** 500
+        assert 2.0 ** -960 <= np.abs(a[nz]).min() and 2.0 ** -960 <= q.min() and q.max() <= 2.0 ** 960
+    P = C.POINTER(C.c_double)
+    assert C.CDLL(str(d / "libt.so")).compare_bits(len(a), a.ctypes.data_as(P), b.ctypes.data_as(P), what) == 0
