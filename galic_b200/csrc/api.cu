@@ -16,6 +16,7 @@
 #include "context.cuh"
 #include "galic_gpu.h"
 #include "kernels.cuh"
+#include "levels.h"
 #include "rep.cuh"
 #include "windows.h"
 
@@ -105,9 +106,8 @@ int check_params(const galic_params_t *p)
 {
   if(!p) return GALIC_ERR_INVALID_ARGUMENT;
   if(p->FG_Nbin < 2 || p->DG_MaxLevel < 1 || p->EG_MaxLevel < 1) return GALIC_ERR_INVALID_ARGUMENT;
-  // eval_fit_mod indexes energy stacks with DG_MaxLevel (main.c:1056) and the
-  // stacks are kept in one CTA's shared memory
-  if(p->DG_MaxLevel != p->EG_MaxLevel || p->DG_MaxLevel > 7) return GALIC_ERR_UNSUPPORTED;
+  // eval_fit_mod indexes energy stacks with DG_MaxLevel (main.c:1056)
+  if(p->DG_MaxLevel != p->EG_MaxLevel || p->DG_MaxLevel > GALIC_MAX_LEVEL) return GALIC_ERR_UNSUPPORTED;
   if(!(p->FG_Rmin > 0) || !(p->FG_Fac > 1) || !(p->DG_Rmin > 0) || !(p->DG_Fac > 1) || !(p->EG_Rmin > 0) ||
      !(p->EG_Fac > 1))
     return GALIC_ERR_INVALID_ARGUMENT;

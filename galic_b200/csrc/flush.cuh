@@ -28,6 +28,7 @@
 
 #include "fixedpoint.cuh"
 #include "kernels.cuh"
+#include "levels.h"
 
 // The four nodes of a cell by parity: node (z, r) lives in slot
 // ((z & 1) << 1) | (r & 1), so that when an orbit moves to a neighbouring cell
@@ -51,6 +52,7 @@ template <int PER_, class T>
 struct WarpQueueT {
   static constexpr int PER = PER_;
   static_assert(PER_ * 32 <= 256, "list entries are bytes");
+  static_assert(1 << (2 * GALIC_MAX_LEVEL) <= 1 << 16, "node indices are 16 bits");
   T val[PER][5][33];             // the node's five sums (33: the five lanes of a record read distinct banks)
   T scale[2][32];                // per lane: {mass field, energy fields} fixed-point factors
   int gbase[32];                 // per lane: first node of its orbit's grid set

@@ -35,12 +35,13 @@
 #include <mutex>
 
 #include "kernels.cuh"
+#include "levels.h"
 
 namespace {
 
 constexpr int kTypes = 3;        // particle types 1..3
 constexpr int kFields = NF_ORBIT;  // m, r, t, q, p
-constexpr int kMaxGrid = 16384;  // DG_MaxLevel <= 7
+constexpr int kMaxGrid = 1 << (2 * GALIC_MAX_LEVEL);
 
 // status words beyond OrbitStatus (the worst code seen wins)
 enum { NOALLOC_OVERFLOW = 3, NOALLOC_INVALID = 4 };
@@ -240,7 +241,7 @@ extern "C" int galic_orbit_responses_noalloc(const galic_params_t *prm, const do
      !(prm->EG_Fac > 1))
     return GALIC_ERR_INVALID_ARGUMENT;
   const int L = prm->DG_MaxLevel;
-  if(L > 7) return GALIC_ERR_BUDGET;  // 4^L bins per grid must fit the fixed scratch array
+  if(L > GALIC_MAX_LEVEL) return GALIC_ERR_BUDGET;  // 4^L bins per grid must fit the fixed scratch array
   const int G = 1 << (2 * L);
   int dev = 0;
   if(cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return GALIC_ERR_NO_DEVICE;

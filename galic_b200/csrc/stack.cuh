@@ -1,11 +1,11 @@
 // CTA-cooperative versions of GALIC's stack routines.
 //
 // A stack holds a quadtree pyramid of a 2^L x 2^L grid; level l starts at
-// STACKOFFSET(l,0,0) = (4^l - 1)/3 (allvars.h:160).  One CTA keeps a whole
-// stack in shared memory (L = 7: 21845 doubles, 171 KiB).
+// STACKOFFSET(l,0,0) = (4^l - 1)/3 (allvars.h:160).
 //
-// stack_smooth_cta: smooth_stack (grid.c:1247-1265), level by level, same
-//                   summation order.
+// stack_smooth_cta: smooth_stack (grid.c:1247-1265) of a whole stack in shared
+//                   memory (L = 7: 21845 doubles, 171 KiB), level by level,
+//                   same summation order.
 // pyramid_cta:      smoothing and calc_stack_difference[_mod]
 //                   (grid.c:1086-1151).  The reference recurses from the root
 //                   and stops at a node when l == maxlevel or
@@ -17,7 +17,9 @@
 #ifndef GALIC_STACK_CUH
 #define GALIC_STACK_CUH
 
-__device__ __forceinline__ int stack_off(int l) { return ((1 << (2 * l)) - 1) / 3; }
+#include "levels.h"
+
+__host__ __device__ constexpr int stack_off(int l) { return ((1 << (2 * l)) - 1) / 3; }
 
 __device__ __forceinline__ void stack_smooth_cta(double *s, int L)
 {
@@ -72,9 +74,11 @@ __device__ __forceinline__ double stack_leaf(double d1, double d2, double r1, do
 //                      finest, and of the finest whose leaf terms are summed
 template <int W, bool MASS>
 struct Pyramid {
-  double d[W][341], v[W][341], r[341];
+  static constexpr int NODES = stack_off(GALIC_MAX_LEVEL - 2);  // levels 0 .. L - 3
+  double d[W][NODES], v[W][NODES], r[NODES];
 };
 
+static_assert(2 * (GALIC_MAX_LEVEL - 1) <= 12, "the nodes of level L - 1 in Z order");
 __device__ __forceinline__ int z_order_half(int m)  // the even bits of m (12 bits)
 {
   m &= 0x555;
