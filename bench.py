@@ -793,6 +793,10 @@ def reference_arm(args, rank, world):
     sys.path.insert(0, os.path.join(ROOT, "tests"))
     import oracle_lib
 
+    if not oracle_lib.reference_available():
+        print(json.dumps({"impl": "reference", "unavailable": "GALIC's own C is not built here (its source tree is "
+                          "absent); the other arm's cpu_baseline times the restatement and says so"}), flush=True)
+        return
     from galic_b200 import synth
 
     # the workload's set-up geometry from the C restatement: this arm never
@@ -814,7 +818,7 @@ def reference_arm(args, rank, world):
             "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
             "config": workload_config(model), "parallelism": f"{cores} host processes",
             "cpu_baseline": {"value": value, "unit": "orbit-steps/s", "cores": cores,
-                             "kind": "reference" if kind == "reference" else "port", "sample": sample,
+                             "kind": kind, "sample": sample,
                              "cpu": cpu_model()},
             "e2e": {"value": value, "unit": "orbit-steps/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
     print(json.dumps(line), flush=True)
@@ -1018,7 +1022,10 @@ def ours_arm(args, rank, world, local_rank):
             v, kind, cores, orbits, st = cpu_orbit_steps_per_s(model, args.cpu_seconds)
             cpu = {"value": v, "unit": "orbit-steps/s", "cores": cores, "kind": kind,
                    "sample": f"{orbits} orbits ({st} orbit-steps) of this workload, {cores} processes, "
-                             f"~{args.cpu_seconds:.0f} s each", "cpu": cpu_model()}
+                             f"~{args.cpu_seconds:.0f} s each, " +
+                             (f"GALIC's C built {REF_BUILD}" if kind == "reference" else
+                              "this repository's C restatement of it (GALIC's own C is not built here)"),
+                   "cpu": cpu_model()}
         fp64_form = form == GALIC_FORM_FP64
         kern_name = "k_calc_all_fp64" if fp64_form else "k_calc_all_fp32"
         traffic = KERNEL_DRAM_BYTES_PER_ORBIT.get(kern_name)
