@@ -55,7 +55,7 @@ namespace {
 constexpr int kSections = 8;       // FG_SECTIONS (allvars.h:123)
 constexpr int kBits = 21;          // BITS_PER_DIMENSION (allvars.h:213)
 constexpr int kMaxTreeLevel = 30;  // MAX_TREE_LEVEL (forcetree.h:16)
-constexpr int kWalkBlock = 64;     // (256: 12.9 against 12.5 ms a fill, means of two runs)
+constexpr int kWalkBlock = 64;     // (256 is no slower: 12.8 - 13.8 ms a fill, 64 13.0 - 14.6, four runs each)
 
 // Peano-Hilbert state machine of peano.c:226-330: next state (kRot) and key
 // digit (kSub) for each state 0..47 and octant pix = 4*x + 2*y + z.  The
@@ -157,8 +157,6 @@ __global__ void k_keys(int n, const double *__restrict__ pos, double cx, double 
   idx[i] = i;
 }
 
-// force_treeevaluate (forcetree_walk.c:12-222), mode 0, one probe per lane.
-// probes: SoA [3][np] in key order; res: SoA [4][np] (acc x, y, z, pot) * G.
 // 2^-200 <= |x| < 2^200: the operands of the walk's step_sqrt and step_div
 __device__ __forceinline__ bool walk_plain(double x)
 {
@@ -170,6 +168,8 @@ __device__ __noinline__ void walk_divide(double mass, double r2, double r, doubl
   *wp = -mass / r;
 }
 
+// force_treeevaluate (forcetree_walk.c:12-222), mode 0, one probe per lane.
+// probes: SoA [3][np] in key order; res: SoA [4][np] (acc x, y, z, pot) * G.
 // What bounds the walk is FP64 issue and the chains of its square root and two
 // divisions; their general forms end basic blocks with tests of the operands.
 // The step's branch-free ones (same bits in walk_plain's range, the general

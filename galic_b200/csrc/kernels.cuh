@@ -21,11 +21,11 @@ enum { NG_COMMITTED = 10 };
 // 3 CTAs of 128 threads per SM (158 registers, none spilled) run the halo +
 // disk pass in 300 ms; 4 CTAs (128 registers, 110 bytes spilled) take 363 ms and
 // 2 CTAs 302 ms: past 2 warps per scheduler the L1 data stage, the issue slots
-// and the FP64 pipe (72, 66 and 50 % busy) share the limit
+// and the FP64 pipe (64, 58 and 43 % busy at 2.4e5 orbits) share the limit
 #define GALIC_FP64_MIN_BLOCKS 3
 #endif
 #ifndef GALIC_FP32_MIN_BLOCKS
-// 5 CTAs per SM (96 registers, none spilled; 5 x 31 KiB of queues) ran the
+// 5 CTAs per SM (96 registers, 20 bytes spilled; 5 x 31 KiB of queues) ran the
 // FP32 pass 2 % faster than 4 (105 registers); 6 (80 registers, spills) 18 %
 // slower
 #define GALIC_FP32_MIN_BLOCKS 5
@@ -74,7 +74,7 @@ struct FitArgs {
   const double *dgs_distance; // [Nstack]
   double *fit;                // [4][7]
   double *raw;                // [4][5]
-  unsigned *arrived;          // [4], 0 between launches
+  unsigned *arrived;          // [4], 0 between whole fits
   int *firstrun;              // [4]
   double thr_d[4], thr_e[4], MType[4];
   int present[4], tovs[4];
@@ -126,10 +126,13 @@ struct FirstOrbit {
 // Orbits of a dense launch, one thread per orbit (-1: none), spread like
 // FirstOrbit over at least DENSE_WARPS warps where there are that many orbits:
 // such a launch lasts as long as its longest orbits, and those take longer in
-// full warps.  Two windows of 3216 composite orbits (FP32) ran 2 x 17.7 ms in
-// 101 warps each, the construction they belong to 65.2 ms; in 592 warps it ran
-// 55.1, in 1184 52.9, in 1776 53.6 ms, six served jobs 60.4, 53.1, 54.0 and
-// 57.2 ms.
+// full warps.  Measured with the warps filled, with at least 592, 888 and 1184
+// of them (ms): one repetition of 401 particles (802 orbits, halo + disk, level
+// 7, FP32) 13.7, 8.7, 8.7, 8.8; of 101 (halo, level 6, FP64) 7.8, 6.2, 6.2, 6.2;
+// the construction of 6e4 composite particles with two windows of 1608
+// particles (FP32) 45.0, 41.5, 42.0, 41.1; six served jobs 56, 53, 53, 53.
+// Two FP64 windows at once would rather have fewer: of 4020 particles (halo +
+// disk, level 6) 16.8, 16.3, 20.0, 21.0.
 constexpr int DENSE_WARPS = 888;
 __device__ __forceinline__ int dense_orbit(int count)
 {
